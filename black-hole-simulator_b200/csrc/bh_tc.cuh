@@ -174,14 +174,23 @@ __device__ inline uint32_t pack2(uint16_t lo, uint16_t hi) { return (uint32_t)lo
 // the network's inputs from con2prim's preamble p5 = (D, tau, Ssq, Bsq, SB)
 // and r: log D, asinh(tau / D), log(1 + S^2 / D^2), log(1 + B^2 / D),
 // asinh(S.B / D^1.5), log r
+template <int I>
+__device__ inline float feature(const double* p5, double r) {
+    const double D = p5[0], tau = p5[1], Ssq = p5[2], Bsq = p5[3], SB = p5[4];
+    if (I == 0) return (float)log(D);
+    if (I == 1) return (float)asinh(tau / D);
+    if (I == 2) return (float)log1p(Ssq / (D * D));
+    if (I == 3) return (float)log1p(Bsq / D);
+    if (I == 4) return (float)asinh(SB / (D * sqrt(D)));
+    return (float)log(r);
+}
 __device__ inline void features(const double* p5, double r, float* x) {
-    double D = p5[0], tau = p5[1], Ssq = p5[2], Bsq = p5[3], SB = p5[4];
-    x[0] = (float)log(D);
-    x[1] = (float)asinh(tau / D);
-    x[2] = (float)log1p(Ssq / (D * D));
-    x[3] = (float)log1p(Bsq / D);
-    x[4] = (float)asinh(SB / (D * sqrt(D)));
-    x[5] = (float)log(r);
+    x[0] = feature<0>(p5, r);
+    x[1] = feature<1>(p5, r);
+    x[2] = feature<2>(p5, r);
+    x[3] = feature<3>(p5, r);
+    x[4] = feature<4>(p5, r);
+    x[5] = feature<5>(p5, r);
 }
 
 // the network's weights into this CTA's shared memory (all threads)
