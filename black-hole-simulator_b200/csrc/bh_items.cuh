@@ -1135,17 +1135,19 @@ BH_HD inline void ptoc_item(const KP& k, const double* W, const double* r, const
     if (Wd) { Wd[q] = po.lor; Wd[n + q] = po.p; Wd[2 * n + q] = po.h; Wd[3 * n + q] = po.b2; }
 }
 
-BH_HD inline void ctop_item(const KP& k, const double* U, const double* r, const double* th, int64_t n, int64_t q,
-                            double* W, double* Wd, int32_t* status, int32_t* iters, int32_t* path) {
+BH_HD inline Cons ctop_load(const double* U, int64_t n, int64_t q) {
     Cons c;
     c.D = U[q]; c.tau = U[4 * n + q];
     for (int d = 0; d < 3; d++) { c.S[d] = U[(1 + d) * n + q]; c.B[d] = U[(5 + d) * n + q]; }
-    Met mc;
-    met_comp(k.tree, r[q], th[q], mc);
+    return c;
+}
+// the fallback and the primitives of cell q, written out
+BH_HD inline void ctop_finish_item(const KP& k, const double gam[3][3], CtopState& s, int64_t n, int64_t q, double* W,
+                                   double* Wd, int32_t* status, int32_t* iters, int32_t* path) {
     Prim w = {0, 0, {0, 0, 0}, {0, 0, 0}};
     CtopOut co = {0, 0, 0, 0, 0, 0, 0};
     bool dom = false;
-    int ok = ctop(k.gamma, k.maxiter, k.tol, mc, c, w, dom, &co);
+    int ok = ctop_end(k.gamma, k.tol, gam, s, w, dom, &co);
     W[q] = w.rho; W[n + q] = w.eps;
     for (int d = 0; d < 3; d++) { W[(2 + d) * n + q] = w.v[d]; W[(5 + d) * n + q] = w.B[d]; }
     if (Wd) { Wd[q] = co.p; Wd[n + q] = co.T; Wd[2 * n + q] = co.h; Wd[3 * n + q] = co.lor; Wd[4 * n + q] = co.b2; }
@@ -1153,39 +1155,26 @@ BH_HD inline void ctop_item(const KP& k, const double* U, const double* r, const
     if (iters) iters[q] = co.iters;
     if (path) path[q] = co.path;
 }
-
-// ctop with Newton started from xi0[q] (bh_ctop_guess); the outputs of ctop_item
-BH_HD inline void ctop_guess_item(const KP& k, const double* U, const double* r, const double* th, int64_t n,
-                                  int64_t q, const double* xi0, double* W, double* Wd, int32_t* status, int32_t* iters,
-                                  int32_t* path) {
-    Cons c;
-    c.D = U[q]; c.tau = U[4 * n + q];
-    for (int d = 0; d < 3; d++) { c.S[d] = U[(1 + d) * n + q]; c.B[d] = U[(5 + d) * n + q]; }
+// one cell of bh_ctop; xi0 (may be NULL): Newton's start (bh_ctop_guess)
+BH_HD inline void ctop_item(const KP& k, const double* U, const double* r, const double* th, int64_t n, int64_t q,
+                            double* W, double* Wd, int32_t* status, int32_t* iters, int32_t* path,
+                            const double* xi0 = nullptr) {
     Met mc;
     met_comp(k.tree, r[q], th[q], mc);
-    Prim w = {0, 0, {0, 0, 0}, {0, 0, 0}};
-    CtopOut co = {0, 0, 0, 0, 0, 0, 0};
-    bool dom = false;
-    int ok = ctop(k.gamma, k.maxiter, k.tol, mc, c, w, dom, &co, xi0[q]);
-    W[q] = w.rho; W[n + q] = w.eps;
-    for (int d = 0; d < 3; d++) { W[(2 + d) * n + q] = w.v[d]; W[(5 + d) * n + q] = w.B[d]; }
-    if (Wd) { Wd[q] = co.p; Wd[n + q] = co.T; Wd[2 * n + q] = co.h; Wd[3 * n + q] = co.lor; Wd[4 * n + q] = co.b2; }
-    status[q] = dom ? -1 : ok;
-    if (iters) iters[q] = co.iters;
-    if (path) path[q] = co.path;
+    CtopState s;
+    ctop_preamble(mc, ctop_load(U, n, q), s, nullptr);
+    ctop_bracket(k.gamma, xi0 ? xi0[q] : NAN, s);
+    while (ctop_newton(k.gamma, k.maxiter, k.tol, s)) {}
+    ctop_finish_item(k, mc.gam, s, n, q, W, Wd, status, iters, path);
 }
 // the preamble quantities of ctop (D, tau, Ssq, Bsq, SB) of cell q, pre [5][n]
 BH_HD inline void ctop_pre_item(const KP& k, const double* U, const double* r, const double* th, int64_t n, int64_t q,
                                 double* pre) {
-    Cons c;
-    c.D = U[q]; c.tau = U[4 * n + q];
-    for (int d = 0; d < 3; d++) { c.S[d] = U[(1 + d) * n + q]; c.B[d] = U[(5 + d) * n + q]; }
     Met mc;
     met_comp(k.tree, r[q], th[q], mc);
-    Prim w;
-    bool dom = false;
+    CtopState s;
     double p5[5];
-    ctop(k.gamma, 0, k.tol, mc, c, w, dom, nullptr, NAN, p5);   // no Newton step: only the preamble is wanted
+    ctop_preamble(mc, ctop_load(U, n, q), s, p5);
     for (int i = 0; i < 5; i++) pre[i * n + q] = p5[i];
 }
 

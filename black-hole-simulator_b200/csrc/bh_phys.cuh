@@ -330,6 +330,58 @@ using PtocOut = PtocOutT<double>;
 // ======================================================================
 // cons -> prim, conserved::ctop + f_df + cp_bd (physics/conserved.cpp:80-285)
 // ======================================================================
+// ---- correctly rounded division and square root without a branch --------
+// The compiler's FP64 division and square root end in a branch to a path for
+// extreme operands, so several of them run one after the other; in con2prim's
+// residual that chain is most of an iteration.  These round the same (to
+// nearest) for operands whose magnitudes and results stay within 2^+-500 (a
+// zero numerator too), which the caller checks for a whole expression at once:
+//   rcp_rn  a hardware approximation y0 (about 2^-20), one third-order step
+//           y = y0 (1 + e + e^2), e = 1 - b y0, then y + y (1 - b y): the
+//           nearest double to 1/b when y is within an ulp of it (Markstein
+//           1990, IBM J. Res. Dev. 34, 111);
+//   div_by  q = a y, then q + y (a - b q) with the remainder exact by FMA
+//           (same reference); one reciprocal serves several quotients;
+//   sqrt_rn Goldschmidt's iteration on g ~ sqrt(x), h ~ 1 / (2 sqrt(x)) from
+//           a hardware approximation, then g + h (x - g^2) (Markstein).
+// Markstein's step misses 1/b by an ulp where b's significand is all ones
+// (all_ones), which the caller checks too.  A host build takes the C operators.
+#ifdef __CUDA_ARCH__
+BH_HD inline bool all_ones(double b) { return ((__double2hiint(b) | (int)0xfff00000) & __double2loint(b)) == -1; }
+BH_HD inline double rcp_polish(double b, double y) { return fma(fma(-b, y, 1.0), y, y); }
+BH_HD inline double rcp_rn(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    const double e = fma(-b, y, 1.0);
+    return rcp_polish(b, fma(fma(e, e, e), y, y));
+}
+// y: a reciprocal of b, correctly rounded
+BH_HD inline double div_by(double a, double b, double y) {
+    double q = a * y;
+    q = fma(fma(-b, q, a), y, q);
+    // (a zero quotient keeps its sign)
+    const int s = (__double2hiint(a) ^ __double2hiint(b)) & (int)0x80000000;
+    return __hiloint2double((__double2hiint(q) & 0x7fffffff) | s, __double2loint(q));
+}
+// i2: about 1 / (2 sqrt(x)), to a few ulps
+BH_HD inline double sqrt_rn(double x, double& i2) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    double g = x * y, h = 0.5 * y, r = fma(-g, h, 0.5);
+    g = fma(g, r, g); h = fma(h, r, h);
+    r = fma(-g, h, 0.5);
+    g = fma(g, r, g); h = fma(h, r, h);
+    i2 = h;
+    return fma(fma(-g, g, x), h, g);
+}
+#else
+BH_HD inline bool all_ones(double) { return false; }
+BH_HD inline double rcp_polish(double b, double) { return 1.0 / b; }
+BH_HD inline double rcp_rn(double b) { return 1.0 / b; }
+BH_HD inline double div_by(double a, double b, double) { return a / b; }
+BH_HD inline double sqrt_rn(double x, double& i2) { i2 = 0.5 / sqrt(x); return sqrt(x); }
+#endif
+
 BH_HD inline double f_df(double gamma, double xi, double Ssq, double Bsq, double SB,
                                        double Dn, double taun, double& df) {
     double Yi = SB * SB;
@@ -388,8 +440,168 @@ BH_HD inline double fres(double gamma, double xi, double Ssq, double Bsq, double
     double d;
     return f_df(gamma, xi, Ssq, Bsq, SB, Dn, taun, d);
 }
+// f_df's own operations in its order, with the divisions and the square root
+// above; false (nothing set) where an operand may leave their range.  `sane`
+// is fdf_sane of the cell.  The reciprocal variants have one division and
+// one square root in f_df and keep it.
+BH_HD inline bool fdf_sane(double Ssq, double Bsq, double SB, double Dn) {
+    return (Ssq == 0.0 || (Ssq >= 1e-40 && Ssq <= 1e40)) && (Bsq == 0.0 || (Bsq >= 1e-40 && Bsq <= 1e18)) &&
+           (SB == 0.0 || (fabs(SB) >= 1e-20 && fabs(SB) <= 1e20)) && Dn >= 1e-30 && Dn <= 1e18;
+}
+BH_HD inline bool fdf_fast(double gamma, double xi, double Ssq, double Bsq, double SB, double Dn, double taun,
+                           bool sane, double& f, double& df) {
+    if (!sane || !(xi >= 1e-15 && xi <= 1e18)) return false;
+    const double Yi = SB * SB, K = Bsq, X = xi * xi, xipK = xi + K;
+    const double N = Ssq * X + Yi * (2.0 * xi + K), Dv = X + xipK * xipK;
+    if (all_ones(Dv)) return false;
+    const double vsq = div_by(N, Dv, rcp_rn(Dv));
+    if (vsq >= 1.0) { f = 1e30; df = 0.0; return true; }
+    const double om = 1.0 - vsq, ltz2 = rcp_rn(om);   // om in [2^-53, 1]
+    double i2l;
+    const double ltz = sqrt_rn(ltz2, i2l);
+    const double il = rcp_polish(ltz, 2.0 * i2l), il2 = rcp_polish(ltz2, om);
+    const double rho = div_by(Dn, ltz, il);
+    const double G = gamma - 1.0, gg = G / gamma;
+    const double p = gg * (div_by(xi, ltz2, il2) - rho);
+    const double iX = rcp_rn(X);
+    const double pstar = p + div_by(K, 2 * ltz2, 0.5 * il2) + div_by(Yi, 2 * X, 0.5 * iX);
+    const double dN = 2.0 * Ssq * xi + 2.0 * Yi;
+    const double dM = 2.0 * xi * xipK * xipK + 2.0 * X * X;
+    const double Mq = X * xipK * xipK, M2 = Mq * Mq;
+    const double dvv = div_by(dN * Mq - dM * N, M2, rcp_rn(M2));
+    const double l4 = ltz2 * ltz2, xX = xi * X;
+    if (!(dvv == 0.0 || (fabs(dvv) >= 1e-100 && fabs(dvv) <= 1e100)) || all_ones(om) || all_ones(ltz) ||
+        all_ones(ltz2) || all_ones(X) || all_ones(M2) || all_ones(l4) || all_ones(xX))
+        return false;
+    if (p < 0.0 || rho < 0.0) { f = 1e32; df = 0.0; return true; }
+    f = xi - taun - Dn - pstar;
+    const double il4 = rcp_polish(l4, il2 * il2);
+    const double dltz2 = ltz2 * ltz2 * dvv;
+    const double dltz = div_by(dltz2, 2.0 * ltz, 0.5 * il);
+    const double dp = gg * (il2 - div_by(xi * dltz2, l4, il4) + div_by(Dn * dltz, ltz2, il2));
+    const double ixX = rcp_polish(xX, xi * iX * iX);
+    const double dpstar = dp - div_by(K * dltz2, 2.0 * ltz2 * ltz2, 0.5 * il4) - div_by(Yi, xX, ixX);
+    df = 1 - dpstar;
+    return true;
+}
+
+// ---- the sign of the residual ------------------------------------------
+// Bracketing reads only the residual's sign: the growth of con2prim's
+// bracket, and all but the two end values of the Brent fallback (A7: fa and
+// fb are never updated, so an iteration's f(s) only decides which end moves).
+// fsgn returns a number of the sign of fres(xi): +-1 where a cheaper
+// evaluation is certain of it, else fres(xi) itself.  The cheaper one forms
+//   f = xi - tau - D - [g (xi om - D sqrt(om)) + K om / 2 + Yi / (2 X)],
+// om = 1 - v^2, g = (gamma - 1) / gamma, from one reciprocal and one
+// reciprocal square root (hardware approximations refined by Newton's
+// iteration), against six divisions and a square root in fres.  Both round
+// every operation by an ulp or two of its terms; the margin err bounds 64
+// roundings (2^-53 each) of every term, om's (relative to the magnitude A
+// of v^2's two terms) carried through xi om, D sqrt(om) and K om.  Outside
+// it the signs agree, and near om = 0 or p = 0, where fres takes its
+// constant branches (v^2 >= 1 and p < 0 count as positive), the decision
+// needs the same margin.  Anything irregular (NaN, overflow, xi or D not
+// positive) goes to fres.
+//   Bound: FP64 latency of the con2prim kernels.  The reciprocal variants
+// keep fres, which has one division and one square root there.
+BH_HD inline double rcp_near(double x) {   // 1/x within a few ulps, x normal
+#ifdef __CUDA_ARCH__
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    y = fma(y, fma(-x, y, 1.0), y);
+    return fma(y, fma(-x, y, 1.0), y);
+#else
+    return 1.0 / x;
+#endif
+}
+BH_HD inline double sqrt_near(double x) {   // sqrt(x) within a few ulps, x normal
+#ifdef __CUDA_ARCH__
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    y = fma(0.5 * y, fma(-x * y, y, 1.0), y);
+    y = fma(0.5 * y, fma(-x * y, y, 1.0), y);
+    return x * y;
+#else
+    return sqrt(x);
+#endif
+}
+// At x < 0 the residual is positive wherever it is a number: p is a sum of
+// two negative terms (or v^2 >= 1), and both branches count as positive.
+// The bounds keep its products finite and its divisors normal.
+BH_HD inline bool positive_below_zero(double gamma, double x, double Ssq, double Bsq, double SB, double D) {
+    return x < -1e-100 && x > -1e152 && x * x * (1.0 + fabs(Ssq)) < 1e304 && D > 0.0 && D < 1e100 && gamma > 1.0 &&
+           fabs(SB) < 1e50 && fabs(Bsq) < 1e100;
+}
+BH_HD inline double fsgn(double gamma, double xi, double Ssq, double Bsq, double SB, double Dn, double taun) {
+    if (positive_below_zero(gamma, xi, Ssq, Bsq, SB, Dn)) return 1.0;
+#ifndef BH_RCP
+    const double U64 = 64.0 * 1.1102230246251565e-16;
+    const double Yi = SB * SB, K = Bsq, X = xi * xi, xK = xi + K, Dv = X + xK * xK, XD = X * Dv;
+    if (XD > 1e-280 && XD < 1e300 && xi > 0.0 && Dn > 0.0) {
+        const double r = rcp_near(XD), iDv = X * r, hX = 0.5 * Dv * r;   // 1 / Dv, 1 / (2 X)
+        const double n1 = Ssq * X, n2 = Yi * (2.0 * xi + K);
+        const double om = 1.0 - (n1 + n2) * iDv, A = 1.0 + (fabs(n1) + fabs(n2)) * iDv;
+        const double dom = U64 * A;
+        if (om < -dom) return 1.0;    // v^2 >= 1
+        if (om > 4.0 * dom) {
+            const double g = (gamma - 1.0) / gamma, s = sqrt_near(om), Ds = Dn * s, xo = xi * om;
+            // om's error in xi om and D sqrt(om) (d sqrt = dom / (2 sqrt), taken twice as large), and the roundings
+            const double e1 = g * (dom * (xi + Dn * rcp_near(s)) + U64 * (xo + Ds));
+            const double p = g * (xo - Ds);
+            if (p < -e1) return 1.0;   // fres's p < 0
+            if (p > e1) {
+                const double y = Yi * hX, f = xi - taun - Dn - (p + 0.5 * K * om + y);
+                const double err = e1 + U64 * (xi + fabs(taun) + Dn + y) + 0.5 * fabs(K) * (dom + U64 * om);
+                if (f > err) return 1.0;
+                if (f < -err) return -1.0;
+            }
+        }
+    }
+#endif
+    return fres(gamma, xi, Ssq, Bsq, SB, Dn, taun);
+}
+// fsgn for many points of one cell: the parts that do not depend on xi are
+// formed once, and the margin is a plain 1e-11 of the terms' magnitudes (far
+// above 64 roundings while om >= 1e-4: om's error is under 2e-14 then, D
+// sqrt(om)'s under 1e-12 D).  With S^2, B^2 >= 0 (sane) v^2's terms and om
+// are within [0, 1].  Falls back to fsgn.
+struct FSgn {
+    double g, hK, c0, c1;
+    bool on;
+};
+BH_HD inline FSgn fsgn_of(double gamma, double Ssq, double Bsq, double SB, double D, double tau) {
+    FSgn q;
+    q.g = (gamma - 1.0) / gamma;
+    q.hK = 0.5 * Bsq;
+    q.c0 = tau + D;
+    q.c1 = fabs(tau) + D + Bsq;
+#ifdef BH_RCP
+    q.on = false;
+#else
+    q.on = gamma > 1.0 && fabs(tau) <= 1e40 && fdf_sane(Ssq, Bsq, SB, D);
+#endif
+    return q;
+}
+BH_HD inline double fsgn_quick(const FSgn& q, double gamma, double xi, double Ssq, double Bsq, double SB, double D,
+                               double tau) {
+    if (q.on && xi >= 1e-15 && xi <= 1e18) {
+        const double X = xi * xi, xK = xi + Bsq, Dv = X + xK * xK, Yi = SB * SB;
+        const double r = rcp_near(X * Dv);
+        const double om = 1.0 - (Ssq * X + Yi * (xi + xK)) * (X * r);
+        if (om >= 1e-4) {
+            const double y = Yi * (0.5 * Dv * r), p = q.g * (xi * om - D * sqrt_near(om));
+            const double f = xi - q.c0 - (p + q.hK * om + y), ep = 1e-11 * (xi + D);
+            if (p < -ep) return 1.0;   // fres's p < 0
+            if (p > ep && fabs(f) > 1e-11 * (xi + q.c1 + y)) return f;
+        } else if (om < -1e-4) {
+            return 1.0;                 // v^2 >= 1
+        }
+    }
+    return fsgn(gamma, xi, Ssq, Bsq, SB, D, tau);
+}
 BH_HD inline bool cp_bd(double gamma, double xa, double xb, double Ssq, double Bsq, double SB, double D,
-                             double tau, double& root, double tol) {
+                             double tau, double& root, double tol, double sa, double sb) {
+    if (sa * sb > 0.0) return false;   // sa, sb: numbers of the sign of fa, fb
     double fa = fres(gamma, xa, Ssq, Bsq, SB, D, tau);
     double fb = fres(gamma, xb, Ssq, Bsq, SB, D, tau);
     if (fa * fb > 0.0) return false;
@@ -402,87 +614,188 @@ BH_HD inline bool cp_bd(double gamma, double xa, double xb, double Ssq, double B
     // its reciprocal is formed here and again after a swap (used by the
     // variants that multiply by reciprocals; the faithful one divides)
     double idfba = 1.0 / (fb - fa);
+#ifndef BH_RCP
+    // the secant point's fraction of the bracket, fb / (fb - fa): it gives s
+    // within a few ulps of the bracket's ends without a division, which is
+    // enough to see most of the steps that are replaced by a bisection
+    double frac = fb * idfba;
+    const FSgn sg = fsgn_of(gamma, Ssq, Bsq, SB, D, tau);
+#endif
     for (int i = 0; i < 100; i++) {
         if (fabs(xb - xa) < tol) { root = xb; return true; }
-        if (fa != fc && fb != fc)
+        bool bisect = false;
+        if (fa != fc && fb != fc) {
             s = (xa * fb * fc) / ((fa - fb) - (fa - fc)) + (xb * fa * fc) / ((fb - fa) - (fb - fc)) +
                 (xc * fa * fb) / ((fc - fa) - (fc - fb));
-        else
-            s = xb - quo(fb * (xb - xa), fb - fa, idfba);
-        bool c1 = !((3 * xa + 4) / 4 < s && s < xb);
-        bool c2 = mflag && fabs(s - xb) >= fabs(xb - xc) / 2;
-        bool c3 = !mflag && fabs(s - xb) >= fabs(xc - d) / 2;
-        if (c1 || c2 || c3) { s = (xa + xb) / 2; mflag = true; }
-        else mflag = false;
-        double fs = fres(gamma, s, Ssq, Bsq, SB, D, tau);
+        } else {
+#ifndef BH_RCP
+            // s lies within m of sn; where the tests below then hold whatever
+            // s is, s itself (a division) is not needed: with xb the lower
+            // end and frac >= 0, s >= xb (c1); frac no number: nor is s
+            bisect = frac != frac || (frac >= 0.0 && xb < xa);
+            if (!bisect) {
+                const double h = frac * (xb - xa), sn = xb - h;
+                const double m = 8.0 * 2.220446049250313e-16 * (fabs(xa) + fabs(xb));
+                const double far = mflag ? fabs(xb - xc) / 2 : fabs(xc - d) / 2;
+                bisect = sn - m > xb || sn + m < (3 * xa + 4) / 4 || fabs(h) - 2.0 * m > far;
+            }
+            if (!bisect)
+#endif
+                s = xb - quo(fb * (xb - xa), fb - fa, idfba);
+        }
+        if (!bisect) {
+            bool c1 = !((3 * xa + 4) / 4 < s && s < xb);
+            bool c2 = mflag && fabs(s - xb) >= fabs(xb - xc) / 2;
+            bool c3 = !mflag && fabs(s - xb) >= fabs(xc - d) / 2;
+            bisect = c1 || c2 || c3;
+        }
+        if (bisect) s = (xa + xb) / 2;
+        mflag = bisect;
+        // f(s) against fa: at s < 0 (tau << 0) f is positive or, where it
+        // overflows, no number, and with fa no number the product is none
+        bool moves_b = false;
+        if (fa == fa && !(fa > 0.0 && s < 0.0 && D > 0.0 && gamma > 1.0)) {
+#ifdef BH_RCP
+            moves_b = fa * fres(gamma, s, Ssq, Bsq, SB, D, tau) < 0.0;
+#else
+            moves_b = fa * fsgn_quick(sg, gamma, s, Ssq, Bsq, SB, D, tau) < 0.0;
+#endif
+        }
         d = xc; xc = xb; fc = fb;
-        if (fa * fs < 0.0) xb = s;
+        if (moves_b) xb = s;
         else xa = s;
         if (fabs(fa) < fabs(fb)) {
             double t = xa; xa = xb; xb = t; t = fa; fa = fb; fb = t;
             idfba = 1.0 / (fb - fa);
+#ifndef BH_RCP
+            frac = fb * idfba;
+#endif
         }
     }
     return false;
 }
 
 struct CtopOut { double p, T, h, lor, b2; int iters, path; };
-// returns 1 ok / 0 failed; *domain set where the reference throws
-// xi0: Newton's start where it lies strictly inside the bracket (the learned
-// guess; NaN, the default, keeps the reference's midpoint); pre[5] (may be
-// null) receives D, tau, Ssq, Bsq, SB of the preamble, and with maxiter = 0
-// ctop returns right after it (pv and co are then not written)
-BH_HD inline int ctop(double gamma, int maxiter, double tol, const Met& mc, const Cons& cv, Prim& pv,
-                           bool& domain, CtopOut* co = nullptr, double xi0 = NAN, double* pre = nullptr) {
+
+// conserved::ctop in three parts, so that a kernel can let a thread take up
+// another cell between Newton steps (k_ctop_refill): begin (the preamble and
+// the bracket), newton (one iteration), end (the fallback and the primitives).
+struct CtopState {
+    double D, tau, B[3], Bu[3], Su[3], Bsq, Ssq, SB;
+    double xi_l, xi_h, xi;
+    double sl, sh;      // numbers of the residual's sign at xi_l and xi_h
+    double seen;        // cycle detection: a past iterate,
+    int since, renew;   // the steps since it and until it is renewed
+    int i, it;          // the loop's index, iterations counted
+    bool nr_ok, conv, sane;
+};
+// Above an x where x (1 - g) outweighs tau + D + K / 2 + Yi / (2 x^2), with
+// S^2, B^2 >= 0 (so that 0 <= v^2 and om <= 1), the residual
+//   f(x) = x - tau - D - [g (x om - D sqrt(om)) + K om / 2 + Yi / (2 x^2)]
+// is positive, and stays so for every larger x (the constant branches
+// v^2 >= 1 and p < 0 are positive too): there the bracket's growth needs no
+// evaluation.  The 1e-9 slack is far above the residual's rounding.
+BH_HD inline bool positive_above(double gamma, double x, double Ssq, double Bsq, double SB, double D, double tau) {
+    const double g = (gamma - 1.0) / gamma;
+    return D > 0.0 && D < 1e40 && Ssq >= 0.0 && Bsq >= 0.0 && x > 1e-30 && x < 1e48 &&
+           x * (1.0 - g) * (1.0 - 1e-9) > (fabs(tau) + D + 0.5 * Bsq) * (1.0 + 1e-9) + SB * SB / (x * x);
+}
+// pre[5] (may be null) receives D, tau, Ssq, Bsq, SB of the preamble; xi0:
+// Newton's start where it lies strictly inside the bracket (the learned
+// guess; NaN keeps the reference's midpoint)
+BH_HD inline void ctop_preamble(const Met& mc, const Cons& cv, CtopState& s, double* pre) {
     double sg = mc.sqrtdetgam, isg = 1.0 / sg;
-    double D = quo(cv.D, sg, isg);
-    double tau = quo(cv.tau, sg, isg);
+    s.D = quo(cv.D, sg, isg);
+    s.tau = quo(cv.tau, sg, isg);
     // conserved.cpp:144-150 reads B[j], S[j] for j > i before they are
     // assigned; those reads are zero here (the reference's value on a clean stack)
-    double B[3] = {0.0, 0.0, 0.0}, S[3] = {0.0, 0.0, 0.0};
-    double Bu[3], Su[3];
+    double S[3] = {0.0, 0.0, 0.0};
+    s.B[0] = s.B[1] = s.B[2] = 0.0;
     double Bsq = 0.0, Ssq = 0.0, SB = 0.0;
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-        B[i] = quo(cv.B[i], sg, isg);
+        s.B[i] = quo(cv.B[i], sg, isg);
         S[i] = quo(cv.S[i], sg, isg);
-        Bu[i] = mc.gam_inv[i][2] * B[2];     // the inner j-loop assigns; j = 2 survives
-        Su[i] = mc.gam_inv[i][2] * S[2];
-        Ssq += S[i] * Su[i];
-        Bsq += B[i] * Bu[i];
-        SB += S[i] * Bu[i];
+        s.Bu[i] = mc.gam_inv[i][2] * s.B[2];     // the inner j-loop assigns; j = 2 survives
+        s.Su[i] = mc.gam_inv[i][2] * S[2];
+        Ssq += S[i] * s.Su[i];
+        Bsq += s.B[i] * s.Bu[i];
+        SB += S[i] * s.Bu[i];
     }
-    if (pre) {
-        pre[0] = D; pre[1] = tau; pre[2] = Ssq; pre[3] = Bsq; pre[4] = SB;
-        if (maxiter == 0) return 0;   // only the preamble was asked for
-    }
+    s.Ssq = Ssq; s.Bsq = Bsq; s.SB = SB;
+    if (pre) { pre[0] = s.D; pre[1] = s.tau; pre[2] = Ssq; pre[3] = Bsq; pre[4] = SB; }
+}
+BH_HD inline void ctop_bracket(double gamma, double xi0, CtopState& s) {
+    const double D = s.D, tau = s.tau, Ssq = s.Ssq, Bsq = s.Bsq, SB = s.SB;
     double xi_l = D;
     double xi_h = tau + D + Bsq / 2.0 + 1e3;
-    double fl = fres(gamma, xi_l, Ssq, Bsq, SB, D, tau);
-    double fh = fres(gamma, xi_h, Ssq, Bsq, SB, D, tau);
+    // (only the signs of these values are read)
+    double fl = fsgn(gamma, xi_l, Ssq, Bsq, SB, D, tau);
+    double fh = fsgn(gamma, xi_h, Ssq, Bsq, SB, D, tau);
+    s.sl = fl;
+    s.sh = fh;
     while (fl * fh > 0.0 && xi_h < 1e8 * D) {
         xi_h *= 2.0;
-        fl = fres(gamma, xi_h, Ssq, Bsq, SB, D, tau);
+        if (fh > 0.0 && positive_above(gamma, xi_h, Ssq, Bsq, SB, D, tau)) {
+            while (xi_h < 1e8 * D) xi_h *= 2.0;
+            s.sh = 1.0;
+            break;
+        }
+        // a negative end, from tau << 0, runs away until f overflows: whole
+        // powers of two at once while that stays short of it
+        if (fh > 0.0 && xi_h < -1e-100)
+            for (double j = 0x1p256; j > 2.0; j = sqrt(j))   // 2^256, 2^128, .. 2^4
+                if (positive_below_zero(gamma, xi_h * j, Ssq, Bsq, SB, D)) xi_h *= j;
+        s.sh = fl = fsgn(gamma, xi_h, Ssq, Bsq, SB, D, tau);
     }
-    double xi = (xi_l + xi_h) / 2.0;
-    if (isfinite(xi0) && xi0 > xi_l && xi0 < xi_h) xi = xi0;
-    bool nr_ok = true, conv = false;
-    int it = 0;
-    for (int i = 0; i < maxiter; i++) {
-        double dF;
-        double F = f_df(gamma, xi, Ssq, Bsq, SB, D, tau, dF);
-        it = i + 1;
-        if (fabs(F) < tol) { conv = true; break; }
-        if (fabs(dF) < 1e-30) { nr_ok = false; break; }
-        double xin = xi - F / dF;
-        if (xin < xi_l || xin > xi_h) { nr_ok = false; break; }
-        xi = xin;
+    s.xi_l = xi_l; s.xi_h = xi_h;
+    s.xi = (xi_l + xi_h) / 2.0;
+    if (isfinite(xi0) && xi0 > xi_l && xi0 < xi_h) s.xi = xi0;
+    s.nr_ok = true; s.conv = false;
+    s.sane = fdf_sane(Ssq, Bsq, SB, D);
+    s.i = 0; s.it = 0;
+    // Where rounding keeps |F| above tol, the iterates end in a cycle, which
+    // the reference walks until maxiter.  An iterate is a function of the one
+    // before alone, so once one repeats (compared with a past iterate that is
+    // renewed at every power of two: Brent 1980's cycle detection), whole
+    // periods are skipped: the same last iterate and count.
+    s.seen = NAN; s.since = 0; s.renew = 1;
+}
+// one Newton iteration; false when the loop has ended
+BH_HD inline bool ctop_newton(double gamma, int maxiter, double tol, CtopState& s) {
+    if (s.i >= maxiter) return false;
+    double F, dF;
+#ifdef BH_RCP
+    F = f_df(gamma, s.xi, s.Ssq, s.Bsq, s.SB, s.D, s.tau, dF);
+#else
+    if (!fdf_fast(gamma, s.xi, s.Ssq, s.Bsq, s.SB, s.D, s.tau, s.sane, F, dF))
+        F = f_df(gamma, s.xi, s.Ssq, s.Bsq, s.SB, s.D, s.tau, dF);
+#endif
+    s.it = s.i + 1;
+    if (fabs(F) < tol) { s.conv = true; return false; }
+    if (fabs(dF) < 1e-30) { s.nr_ok = false; return false; }
+    double xin = s.xi - F / dF;
+    if (xin < s.xi_l || xin > s.xi_h) { s.nr_ok = false; return false; }
+    s.xi = xin;
+    s.since++;
+    if ((xin == s.seen && xin != 0.0) || xin != xin) {   // (NaN stays NaN)
+        s.i += (maxiter - 1 - s.i) / s.since * s.since;
+        s.it = s.i + 1;
     }
-    int path = conv ? 0 : 1;
-    if (!nr_ok) {
+    if (s.since == s.renew) { s.seen = xin; s.since = 0; s.renew *= 2; }
+    s.i++;
+    return true;
+}
+// returns 1 ok / 0 failed; *domain set where the reference throws
+BH_HD inline int ctop_end(double gamma, double tol, const double gam[3][3], CtopState& s, Prim& pv, bool& domain,
+                          CtopOut* co) {
+    const double Bsq = s.Bsq, Ssq = s.Ssq, SB = s.SB, D = s.D;
+    double xi = s.xi;
+    int path = s.conv ? 0 : 1;
+    if (!s.nr_ok) {
         double xib;
-        if (!cp_bd(gamma, xi_l, xi_h, Ssq, Bsq, SB, D, tau, xib, tol)) {
-            if (co) { co->iters = it; co->path = 3; }
+        if (!cp_bd(gamma, s.xi_l, s.xi_h, Ssq, Bsq, SB, D, s.tau, xib, tol, s.sl, s.sh)) {
+            if (co) { co->iters = s.it; co->path = 3; }
             return 0;
         }
         path = 2;
@@ -504,25 +817,36 @@ BH_HD inline int ctop(double gamma, int maxiter, double tol, const Met& mc, cons
     double ixpQ = 1.0 / xpQ;
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-        pv.v[i] = quo(Su[i] + (SB / xi) * Bu[i], xpQ, ixpQ);
-        pv.B[i] = B[i];
+        pv.v[i] = quo(s.Su[i] + (SB / xi) * s.Bu[i], xpQ, ixpQ);
+        pv.B[i] = s.B[i];
     }
     if (co) {
         double Blow[3] = {0.0, 0.0, 0.0};
 #pragma unroll
         for (int i = 0; i < 3; i++)
 #pragma unroll
-            for (int j = 0; j < 3; j++) Blow[i] += mc.gam[i][j] * B[j];
+            for (int j = 0; j < 3; j++) Blow[i] += gam[i][j] * s.B[j];
         double Bv = 0.0;
 #pragma unroll
         for (int i = 0; i < 3; i++)
 #pragma unroll
-            for (int j = 0; j < 3; j++) Bv += Blow[i] * mc.gam[i][j] * pv.v[j];
+            for (int j = 0; j < 3; j++) Bv += Blow[i] * gam[i][j] * pv.v[j];
         co->b2 = (Bv * Bv + Bsq) / ltz2;
-        co->p = p; co->h = hh; co->T = T; co->lor = ltz; co->iters = it; co->path = path;
+        co->p = p; co->h = hh; co->T = T; co->lor = ltz; co->iters = s.it; co->path = path;
     }
     if (pv.rho <= 0.0 || pv.eps <= 0.0 || p <= 0.0) return 0;
     return 1;
+}
+// the whole; with pre set and maxiter = 0 it returns right after the
+// preamble (pv and co are then not written)
+BH_HD inline int ctop(double gamma, int maxiter, double tol, const Met& mc, const Cons& cv, Prim& pv,
+                           bool& domain, CtopOut* co = nullptr, double xi0 = NAN, double* pre = nullptr) {
+    CtopState s;
+    ctop_preamble(mc, cv, s, pre);
+    if (pre && maxiter == 0) return 0;   // only the preamble was asked for
+    ctop_bracket(gamma, xi0, s);
+    while (ctop_newton(gamma, maxiter, tol, s)) {}
+    return ctop_end(gamma, tol, mc.gam, s, pv, domain, co);
 }
 
 // floor state amrtree::pvfs (grid.cpp:133-146; constants grid.hpp:140-143)

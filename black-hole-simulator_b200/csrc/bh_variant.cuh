@@ -64,13 +64,54 @@ __global__ void k_metric(KP k, const double* r, const double* th, int64_t n, dou
 __global__ void k_ptoc(KP k, const double* W, const double* r, const double* th, int64_t n, double* U, double* Wd) {
     BATCH; ptoc_item(k, W, r, th, n, q, U, Wd, nullptr);
 }
-__global__ void k_ctop(KP k, const double* U, const double* r, const double* th, int64_t n, double* W, double* Wd,
-                       int32_t* st, int32_t* it, int32_t* pa) {
-    BATCH; ctop_item(k, U, r, th, n, q, W, Wd, st, it, pa);
-}
-__global__ void k_ctop_guess(KP k, const double* U, const double* r, const double* th, int64_t n, const double* xi0,
-                             double* W, double* Wd, int32_t* st, int32_t* it, int32_t* pa) {
-    BATCH; ctop_guess_item(k, U, r, th, n, q, xi0, W, Wd, st, it, pa);
+// con2prim of a batch: a warp takes `per_warp` consecutive cells, and a lane
+// whose cell's Newton iteration has ended takes the warp's next cell, so that
+// the lanes iterate together although the counts differ.  Cells are finished
+// and taken up once CT_REFILL lanes wait (both have work of their own, done
+// by the waiting lanes only), and at the end when all do.  Each cell's own
+// operations are those of ctop_item.
+//   Bound: FP64 latency and issue (the stress batch's 2M cells read and write
+// 0.4 GB).  A cell takes 4.5 Newton iterations in the mean, the slowest of 32
+// about 30, and 0.05 % of them run to maxiter, which is the time of a small
+// batch.  One resident wave shares the cells evenly, so that every warp has
+// many to refill from.  2M cells, one thread per cell 4.4 ms, this form 1.56
+// ms (12 / 20 waiting lanes and 3 / 4 CTAs per SM: 1.84, 1.66, -, 1.56).
+constexpr int CT_REFILL = 20, CT_CTAS = 4;
+__global__ void __launch_bounds__(TPB, CT_CTAS) k_ctop(KP k, const double* U, const double* r, const double* th, int64_t n,
+                                               const double* xi0, double* W, double* Wd, int32_t* st, int32_t* it,
+                                               int32_t* pa, int64_t per_warp) {
+    const int lane = threadIdx.x & 31;
+    const int64_t first = ((int64_t)blockIdx.x * (TPB / 32) + (threadIdx.x >> 5)) * per_warp;
+    const int64_t last = first + per_warp < n ? first + per_warp : n;
+    int64_t next = first, q = -1;   // the warp's next cell; this lane's cell
+    bool run = false;
+    CtopState s;
+    double g11 = 0.0, g13 = 0.0, g22 = 0.0, g33 = 0.0;
+    for (;;) {
+        const unsigned idle = __ballot_sync(0xffffffffu, !run);
+        if (idle == 0xffffffffu || (next < last && __popc(idle) >= CT_REFILL)) {
+            if (!run) {
+                if (q >= 0) {
+                    const double gam[3][3] = {{g11, 0.0, g13}, {0.0, g22, 0.0}, {g13, 0.0, g33}};
+                    ctop_finish_item(k, gam, s, n, q, W, Wd, st, it, pa);
+                }
+                q = next + __popc(idle & ((1u << lane) - 1u));
+                if (q < last) {
+                    Met mc;
+                    met_comp(k.tree, r[q], th[q], mc);
+                    g11 = mc.gam[0][0]; g13 = mc.gam[0][2]; g22 = mc.gam[1][1]; g33 = mc.gam[2][2];
+                    ctop_preamble(mc, ctop_load(U, n, q), s, nullptr);
+                    ctop_bracket(k.gamma, xi0 ? xi0[q] : NAN, s);
+                    run = true;
+                } else {
+                    q = -1;
+                }
+            }
+            next += __popc(idle);
+            if (__ballot_sync(0xffffffffu, run) == 0) return;
+        }
+        if (run) run = ctop_newton(k.gamma, k.maxiter, k.tol, s);
+    }
 }
 __global__ void k_ctop_pre(KP k, const double* U, const double* r, const double* th, int64_t n, double* pre) {
     BATCH; ctop_pre_item(k, U, r, th, n, q, pre);
@@ -106,14 +147,10 @@ __global__ void __launch_bounds__(bh_tc::ROWS, 4)
         float xn[bh_tc::NI];
         bool valid = false;
         if (in) {
-            Cons c;
-            c.D = U[q]; c.tau = U[4 * n + q];
-            for (int d = 0; d < 3; d++) { c.S[d] = U[(1 + d) * n + q]; c.B[d] = U[(5 + d) * n + q]; }
             Met mc;
             met_comp(k.tree, r[q], th[q], mc);
-            Prim w0;
-            bool dom0 = false;
-            ctop(k.gamma, 0, k.tol, mc, c, w0, dom0, nullptr, NAN, p5);   // the preamble only
+            CtopState cs;
+            ctop_preamble(mc, ctop_load(U, n, q), cs, p5);
             float x[bh_tc::NI];
             bh_tc::features(p5, r[q], x);
             valid = true;
@@ -341,6 +378,20 @@ inline bool bad_pool(const bh_pool* p) {
 }
 // entries of pool->all: the patches the flux/CT/update/floors kernels visit
 inline int nall(const bh_pool* p) { return p->nall > 0 ? p->nall : p->npatch; }
+inline int ctop_launch(const bh_params* P, const double* U, const double* r, const double* th, int64_t n,
+                       const double* xi0, double* W, double* Wd, int32_t* status, int32_t* iters, int32_t* path,
+                       void* stream) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return BH_ECUDA;
+    // one wave: the CTAs that are resident at once share the cells evenly
+    const int64_t most = (int64_t)sms * CT_CTAS, cta = (n + TPB - 1) / TPB;
+    const int64_t grid = cta < most ? cta : most, warps = grid * (TPB / 32);
+    k_ctop<<<(unsigned)grid, TPB, 0, S(stream)>>>(kp_of(P), U, r, th, n, xi0, W, Wd, status, iters, path,
+                                                (n + warps - 1) / warps);
+    return launched();
+}
 inline dim3 grid2(int items, int npatch, int z = 1) { return dim3((items + TPB - 1) / TPB, npatch, z); }
 
 // ---- launch bounds chosen by the autotuner --------------------------------
@@ -397,8 +448,7 @@ int ctop(const bh_params* P, const double* U, const double* r, const double* th,
             int32_t* status, int32_t* iters, int32_t* path, void* stream) {
     if (!P || n < 0 || (n > 0 && !status)) return BH_EINVAL;
     if (n == 0) return BH_OK;
-    k_ctop<<<(unsigned)((n + TPB - 1) / TPB), TPB, 0, S(stream)>>>(kp_of(P), U, r, th, n, W, Wd, status, iters, path);
-    return launched();
+    return ctop_launch(P, U, r, th, n, nullptr, W, Wd, status, iters, path, stream);
 }
 int hlld(const bh_params* P, const double* WL, const double* WR, const double* UL, const double* UR,
             const double* r, const double* th, int32_t dim, int64_t n, double* F, double* ctspeed, void* stream) {
@@ -509,9 +559,7 @@ int ctop_guess(const bh_params* P, const double* U, const double* r, const doubl
                double* W, double* Wd, int32_t* status, int32_t* iters, int32_t* path, void* stream) {
     if (!P || n < 0 || (n > 0 && (!U || !r || !th || !xi0 || !W || !status))) return BH_EINVAL;
     if (n == 0) return BH_OK;
-    k_ctop_guess<<<(unsigned)((n + TPB - 1) / TPB), TPB, 0, S(stream)>>>(kp_of(P), U, r, th, n, xi0, W, Wd, status,
-                                                                      iters, path);
-    return launched();
+    return ctop_launch(P, U, r, th, n, xi0, W, Wd, status, iters, path, stream);
 }
 int ctop_learned(const bh_params* P, const bh_mlp* m, const double* U, const double* r, const double* th,
                  int64_t n, double* xi0, double* W, double* Wd, int32_t* status, int32_t* iters, int32_t* path,
@@ -539,9 +587,7 @@ int ctop_learned(const bh_params* P, const bh_mlp* m, const double* U, const dou
     k_guess_tc<<<(unsigned)grid, bh_tc::ROWS, 0, S(stream)>>>(kp_of(P), (const __nv_bfloat16*)m->wb,
                                                             m->w + BH_MLP_NPARAM, U, r, th, n, xi0, err);
     if (cudaGetLastError() != cudaSuccess) return BH_ECUDA;
-    k_ctop_guess<<<(unsigned)((n + TPB - 1) / TPB), TPB, 0, S(stream)>>>(kp_of(P), U, r, th, n, xi0, W, Wd, status,
-                                                                      iters, path);
-    return launched();
+    return ctop_launch(P, U, r, th, n, xi0, W, Wd, status, iters, path, stream);
 }
 int ctop_pre(const bh_params* P, const double* U, const double* r, const double* th, int64_t n, double* pre,
              void* stream) {
