@@ -749,7 +749,7 @@ def run_ours(args):
                            "(interior cells' U and W rows 0-4, the blocks' own faces) from pinned host memory in and "
                            "out every step, unpacked and packed on the device",
                     "serial_value": world * zones / (ms_e2e_serial / 1e3), "serial_ms_per_step": ms_e2e_serial},
-            "gpu_launches": (LAUNCHES_PER_STEP + (2 if tune_get("mixed", "split") else 0)) * args.steps,
+            "gpu_launches": (LAUNCHES_PER_STEP + (2 if tune_get("mixed", "split") == 1 else 0)) * args.steps,
             "roofline": {"bound": "hbm", "kernel": f"{kname} ({top})", "achieved": achieved, "peak": peak,
                          "unit": "GB/s", "frac": achieved / peak,
                          "traffic": PROFILED_TRAFFIC.get(top) if args.grid == 128 else None,

@@ -430,7 +430,8 @@ lib.bh_fx_tune_get.restype = C.c_int
 
 
 def tune_set(precision: str, kernel: str, ctas: int):
-    """kernel in TUNE_KERNELS: resident CTAs per SM (1, 3..8); "stage", "split": 0/1."""
+    """kernel in TUNE_KERNELS: resident CTAs per SM (1, 3..8), 0 for the
+    library's rules (the initial choice); "stage", "split": 0/1, 2 by rule."""
     check(lib.bh_fx_tune_set(PRECISIONS[precision], TUNE_KNOBS.index(kernel), ctas), "bh_fx_tune_set")
 
 

@@ -1158,10 +1158,12 @@ inline int fx_grid(const void* fn, int nitem, const bh_fx_grid* g) {
 
 // launch bounds of the heavy kernels: resident 128-thread CTAs per SM asked
 // of ptxas (which caps registers per thread); 1 leaves the choice to ptxas.
-// Chosen per process and variant (bh_fx_tune_set), initially 1.
-int fx_tune_tab[BH_FX_TUNE_N] = {1, 1, 1, 0, 0};
-#define FX_TUNED(kernel, LAUNCH)                                                  \
-    switch (fx_tune_tab[kernel]) {                                                \
+// Chosen per process and variant (bh_fx_tune_set); initially the rules of
+// fx_choose, which follow the grid and the scheme.
+constexpr int FX_AUTO = 0, FX_AUTO_FORM = 2;   // the knobs' "by rule" values
+int fx_tune_tab[BH_FX_TUNE_N] = {FX_AUTO, FX_AUTO, FX_AUTO, FX_AUTO_FORM, FX_AUTO_FORM};
+#define FX_TUNED(choice, LAUNCH)                                                  \
+    switch (choice) {                                                             \
     case 3: LAUNCH(3); break;                                                     \
     case 4: LAUNCH(4); break;                                                     \
     case 5: LAUNCH(5); break;                                                     \
@@ -1170,11 +1172,47 @@ int fx_tune_tab[BH_FX_TUNE_N] = {1, 1, 1, 0, 0};
     case 8: LAUNCH(8); break;                                                     \
     default: LAUNCH(1); break;                                                    \
     }
+namespace {
+// The rules, from kernel times in us on B200 (mixed / FP64; "1" = no cap, the
+// former default), over the 128^3 torus, 96^3 in 32^3 blocks and 512 blocks of
+// 8^3 to 32^3 (lev):
+//   con2prim  7 (mixed), 6: 128^3 237 -> 122 / 337 -> 197, lev 175 -> 105 / 241 -> 149.
+//   fluxes    the stencil staged where the tiles pad the positions by at most
+//             a tenth (blocks of ~100^3 on): 128^3 (8 %) 275 against 292 /
+//             587 against 621 unstaged, 64^3 (16 %) 45 against 42 / 94 against 87.
+//             Resident CTAs 8 in FP32 (128^3 365 -> 275, PPM 540 -> 431);
+//             in FP64 4 staged (697 -> 587) and 5 unstaged (782 -> 621, PPM
+//             1082 -> 856, lev 812 -> 636): more would spill.
+//   update    8 in FP32, 6 in FP64; as its two kernels with edge EMFs in arrays
+//             (lev 243 -> 222 / 312 -> 301) and for FP64 grids of 8192 items
+//             or more (128^3 282 -> 269; below that the second launch costs
+//             more: 16^3 12 -> 14).
+// A grid of up to four items per SM takes no cap: nothing waits for a slot,
+// and a capped kernel's spills only lengthen it (16^3 step 134 -> 144).
+int fx_choose(int kernel, const bh_fx_params* P, const bh_fx_grid* g) {
+    const int set = fx_tune_tab[kernel];
+    constexpr bool F32 = sizeof(FRT) < sizeof(double);
+    const bool staged = fx_tune_tab[BH_FX_TUNE_STAGE] == FX_AUTO_FORM
+                            ? g->nitem_flux > g->nitem_pos && 10 * (int64_t)g->nitem_flux <= 11 * (int64_t)g->nitem_pos
+                            : fx_tune_tab[BH_FX_TUNE_STAGE] == 1;
+    const int few = 4 * fx_sms();   // work items
+    switch (kernel) {
+    case BH_FX_TUNE_STAGE: return staged && g->nitem_flux && P->limiter != fx::FX_PPM;
+    case BH_FX_TUNE_SPLIT:
+        return set != FX_AUTO_FORM ? set : (g->E || (!F32 && g->nitem_cell >= 8192));
+    case BH_FX_TUNE_C2P: return set != FX_AUTO ? set : (g->nitem_cell <= few ? 1 : (F32 ? 7 : 6));
+    case BH_FX_TUNE_FLUX:
+        if (set != FX_AUTO) return set;
+        return g->nitem_pos <= few ? 1 : (F32 ? 8 : (staged && P->limiter != fx::FX_PPM ? 4 : 5));
+    default: return set != FX_AUTO ? set : (g->nitem_cell <= few ? 1 : (F32 ? 8 : 6));
+    }
+}
+}  // namespace
 
 int fx_tune_set(int32_t kernel, int32_t ctas) {
     if (kernel == BH_FX_TUNE_STAGE || kernel == BH_FX_TUNE_SPLIT) {
-        if (ctas != 0 && ctas != 1) return BH_EINVAL;
-    } else if (kernel < 0 || kernel >= BH_FX_TUNE_N || !(ctas == 1 || (ctas >= 3 && ctas <= 8))) {
+        if (ctas < 0 || ctas > FX_AUTO_FORM) return BH_EINVAL;
+    } else if (kernel < 0 || kernel >= BH_FX_TUNE_N || !(ctas == FX_AUTO || ctas == 1 || (ctas >= 3 && ctas <= 8))) {
         return BH_EINVAL;
     }
     fx_tune_tab[kernel] = ctas;
@@ -1192,7 +1230,7 @@ int fx_prims(const bh_fx_params* P, const bh_fx_grid* g, int32_t stage, int32_t 
     if (with_dt) fx::k_fx_dt_init<<<1, 1, 0, fxs(s)>>>(g->dt);
     if (g->nitem_cell) {
 #define L_(M) fx::k_fx_c2p<FRT, FRT, M><<<fx_grid((const void*)fx::k_fx_c2p<FRT, FRT, M>, g->nitem_cell, g), fx::FX_TPB, 0, fxs(s)>>>(p, G, g->items_cell, stage, with_dt, fx_q(g, QS_C2P, g->nitem_cell))
-        FX_TUNED(BH_FX_TUNE_C2P, L_)
+        FX_TUNED(fx_choose(BH_FX_TUNE_C2P, P, g), L_)
 #undef L_
     }
     return fx_launched();
@@ -1213,13 +1251,13 @@ int fx_ghosts(const bh_fx_params* P, const bh_fx_grid* g, int32_t stage, void* s
 int fx_fluxes(const bh_fx_params* P, const bh_fx_grid* g, int32_t stage, void* s) {
     fx::FxPar p = fx::par_of(P);
     fx::Grid G = fx::grid_of(g);
-    if (fx_tune_tab[BH_FX_TUNE_STAGE] && g->nitem_flux && P->limiter != fx::FX_PPM) {
+    if (fx_choose(BH_FX_TUNE_STAGE, P, g)) {
 #define L_(M) fx::k_fx_flux_tile<FRT, FRT, FRT, M><<<fx_grid((const void*)fx::k_fx_flux_tile<FRT, FRT, FRT, M>, g->nitem_flux, g), fx::FX_TPB, 0, fxs(s)>>>(p, G, g->items_flux, stage, fx_q(g, QS_FLUX, g->nitem_flux))
-        FX_TUNED(BH_FX_TUNE_FLUX, L_)
+        FX_TUNED(fx_choose(BH_FX_TUNE_FLUX, P, g), L_)
 #undef L_
     } else if (g->nitem_pos) {
 #define L_(M) fx::k_fx_flux<FRT, FRT, FRT, M><<<fx_grid((const void*)fx::k_fx_flux<FRT, FRT, FRT, M>, g->nitem_pos, g), fx::FX_TPB, 0, fxs(s)>>>(p, G, g->items_pos, stage, fx_q(g, QS_FLUX, g->nitem_pos))
-        FX_TUNED(BH_FX_TUNE_FLUX, L_)
+        FX_TUNED(fx_choose(BH_FX_TUNE_FLUX, P, g), L_)
 #undef L_
     }
     return fx_launched();
@@ -1236,15 +1274,15 @@ int fx_update_parts(const bh_fx_params* P, const bh_fx_grid* g, int32_t stage, i
     if (g->E && g->nitem_pos && g->maxlevel > 0)
         fx::k_fx_emf_fix<<<fx_grid((const void*)fx::k_fx_emf_fix, g->nitem_pos, g), fx::FX_TPB, 0, fxs(s)>>>(
             G, g->items_pos, fx_q(g, QS_EMF_FIX, g->nitem_pos));
-    if (g->nitem_cell && fx_tune_tab[BH_FX_TUNE_SPLIT]) {
+    if (g->nitem_cell && fx_choose(BH_FX_TUNE_SPLIT, P, g)) {
 #define L_(M) fx::k_fx_update<FRT, FRT, FRT, M, 1><<<fx_grid((const void*)fx::k_fx_update<FRT, FRT, FRT, M, 1>, g->nitem_cell, g), fx::FX_TPB, 0, fxs(s)>>>(p, G, g->items_cell, stage, P->cfl, fx_q(g, QS_UPDATE, g->nitem_cell))
-        FX_TUNED(BH_FX_TUNE_UPDATE, L_)
+        FX_TUNED(fx_choose(BH_FX_TUNE_UPDATE, P, g), L_)
 #undef L_
         fx::k_fx_update<FRT, FRT, FRT, 8, 2><<<fx_grid((const void*)fx::k_fx_update<FRT, FRT, FRT, 8, 2>, g->nitem_cell, g), fx::FX_TPB, 0, fxs(s)>>>(
             p, G, g->items_cell, stage, P->cfl, fx_q(g, QS_UPDATE_B, g->nitem_cell));
     } else if (g->nitem_cell) {
 #define L_(M) fx::k_fx_update<FRT, FRT, FRT, M, 3><<<fx_grid((const void*)fx::k_fx_update<FRT, FRT, FRT, M, 3>, g->nitem_cell, g), fx::FX_TPB, 0, fxs(s)>>>(p, G, g->items_cell, stage, P->cfl, fx_q(g, QS_UPDATE, g->nitem_cell))
-        FX_TUNED(BH_FX_TUNE_UPDATE, L_)
+        FX_TUNED(fx_choose(BH_FX_TUNE_UPDATE, P, g), L_)
 #undef L_
     }
     return fx_launched();
