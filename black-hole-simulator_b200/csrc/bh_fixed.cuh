@@ -775,22 +775,67 @@ __global__ void __launch_bounds__(FX_TPB, MINB) k_fx_update(FxPar P, Grid G, con
         const double dt = cfl * G.dt[0];
         if ((PART & 1) && stage == 0 && t == 0 && threadIdx.x == 0) G.dt[1] = dt;
         const double idx = 1.0 / B.dx;
+        // In FP64 everything read of the state goes out first: between the
+        // stores a load waits for the store before it, which may alias, one
+        // round trip to memory per variable (128^3, both halves, stages 0 and 1:
+        // 216 and 230 us at 4 CTAs per SM, before 266 and 272 at its best, 6).  The mixed variant keeps its order: the
+        // compiler contracts the FP32 source by it, and a step's roundings
+        // are to stay.
+        constexpr bool EARLY = sizeof(RT) == sizeof(double);
+        double u0[5], u1[5], b0[3], b1[3];
+        FT div[5];
+        if constexpr (EARLY) {
+            if (PART & 1) {
+#pragma unroll
+                for (int v = 0; v < 5; v++) {
+                    u0[v] = G.U[v * N + c];
+                    if (stage) u1[v] = G.U1[v * N + c];
+                }
+            }
+            if (PART & 2) {
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    b0[d] = G.Bf[d * N + c];
+                    if (stage) b1[d] = G.Bf1[d * N + c];
+                }
+            }
+        }
         if (PART & 1) {
+        const WT* W = (const WT*)G.W;
+        RT w[8];
+        if constexpr (EARLY) {
+#pragma unroll
+            for (int v = 0; v < 8; v++) w[v] = RT(W[v * N + c]);
+#pragma unroll
+            for (int v = 0; v < 5; v++)
+                div[v] = (fget<FT>(G, 0, v, c + si) - fget<FT>(G, 0, v, c)) * FT(idx) +
+                         (fget<FT>(G, 1, v, c + sj) - fget<FT>(G, 1, v, c)) * FT(idx) +
+                         (fget<FT>(G, 2, v, c + sk) - fget<FT>(G, 2, v, c)) * FT(idx);
+        }
         // source at the cell centre from the stage's primitives
         double x[3];
         cell_centre(B, i, j, k, x);
         KSb<RT> mk;
         KSDb<RT> dk;
         cell_geometry<RT>(P, x, mk, dk);
-        const WT* W = (const WT*)G.W;
-        RT w[8];
-        for (int v = 0; v < 8; v++) w[v] = RT(W[v * N + c]);
+        if constexpr (!EARLY)
+            for (int v = 0; v < 8; v++) w[v] = RT(W[v * N + c]);
         RT S[8];
         source<RT>(mk, dk, RT(P.gg), w, S);
         // the flux divergence in the flux type (the differences of
         // neighbouring faces' values are exact in FP32 where they are within
         // a factor of two of each other)
         const FT idf = FT(idx);
+        if constexpr (EARLY) {
+#pragma unroll
+            for (int v = 0; v < 5; v++) {
+                double L = (double)S[v] - (double)div[v];
+                if (stage == 0)
+                    G.U1[v * N + c] = u0[v] + dt * L;
+                else
+                    G.U[v * N + c] = 0.5 * (u0[v] + u1[v] + dt * L);
+            }
+        } else {
         for (int v = 0; v < 5; v++) {
             FT div = (fget<FT>(G, 0, v, c + si) - fget<FT>(G, 0, v, c)) * idf +
                      (fget<FT>(G, 1, v, c + sj) - fget<FT>(G, 1, v, c)) * idf +
@@ -800,6 +845,7 @@ __global__ void __launch_bounds__(FX_TPB, MINB) k_fx_update(FxPar P, Grid G, con
                 G.U1[v * N + c] = G.U[v * N + c] + dt * L;
             else
                 G.U[v * N + c] = 0.5 * (G.U[v * N + c] + G.U1[v * N + c] + dt * L);
+        }
         }
         }
         if (!(PART & 2)) return;
@@ -821,11 +867,18 @@ __global__ void __launch_bounds__(FX_TPB, MINB) k_fx_update(FxPar P, Grid G, con
         const double curl[3] = {(ez[2] - ez[0]) * idx - (ey[2] - ey[0]) * idx,
                                 (ex[2] - ex[0]) * idx - (ez[1] - ez[0]) * idx,
                                 (ey[1] - ey[0]) * idx - (ex[1] - ex[0]) * idx};
+        if constexpr (!EARLY) {
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                b0[d] = G.Bf[d * N + c];
+                if (stage) b1[d] = G.Bf1[d * N + c];
+            }
+        }
         for (int d = 0; d < 3; d++) {
             if (stage == 0)
-                G.Bf1[d * N + c] = G.Bf[d * N + c] - dt * curl[d];
+                G.Bf1[d * N + c] = b0[d] - dt * curl[d];
             else
-                G.Bf[d * N + c] = 0.5 * (G.Bf[d * N + c] + G.Bf1[d * N + c] - dt * curl[d]);
+                G.Bf[d * N + c] = 0.5 * (b0[d] + b1[d] - dt * curl[d]);
         }
         if (i == n - 1) face_update<FT>(G, 0, c + si, si, sj, sk, idx, dt, stage);
         if (j == n - 1) face_update<FT>(G, 1, c + sj, si, sj, sk, idx, dt, stage);
@@ -1183,10 +1236,11 @@ namespace {
 //             Resident CTAs 8 in FP32 (128^3 365 -> 275, PPM 540 -> 431);
 //             in FP64 4 staged (697 -> 587) and 5 unstaged (782 -> 621, PPM
 //             1082 -> 856, lev 812 -> 636): more would spill.
-//   update    8 in FP32, 6 in FP64; as its two kernels with edge EMFs in arrays
-//             (lev 243 -> 222 / 312 -> 301) and for FP64 grids of 8192 items
-//             or more (128^3 282 -> 269; below that the second launch costs
-//             more: 16^3 12 -> 14).
+//   update    8 in FP32, 4 in FP64 (whose early loads fill the registers); as
+//             its two kernels with edge EMFs in arrays (lev 249 -> 210 / 249 ->
+//             248) and on grids of 8192 items, in FP64 2048, or more (128^3
+//             169 -> 166 a stage / 255 -> 223, 64^3 40 -> 38; below that the
+//             second launch costs more: 16^3 12 -> 17).
 // A grid of up to four items per SM takes no cap: nothing waits for a slot,
 // and a capped kernel's spills only lengthen it (16^3 step 134 -> 144).
 int fx_choose(int kernel, const bh_fx_params* P, const bh_fx_grid* g) {
@@ -1199,12 +1253,12 @@ int fx_choose(int kernel, const bh_fx_params* P, const bh_fx_grid* g) {
     switch (kernel) {
     case BH_FX_TUNE_STAGE: return staged && g->nitem_flux && P->limiter != fx::FX_PPM;
     case BH_FX_TUNE_SPLIT:
-        return set != FX_AUTO_FORM ? set : (g->E || (!F32 && g->nitem_cell >= 8192));
+        return set != FX_AUTO_FORM ? set : (g->E || g->nitem_cell >= (F32 ? 8192 : 2048));
     case BH_FX_TUNE_C2P: return set != FX_AUTO ? set : (g->nitem_cell <= few ? 1 : (F32 ? 7 : 6));
     case BH_FX_TUNE_FLUX:
         if (set != FX_AUTO) return set;
         return g->nitem_pos <= few ? 1 : (F32 ? 8 : (staged && P->limiter != fx::FX_PPM ? 4 : 5));
-    default: return set != FX_AUTO ? set : (g->nitem_cell <= few ? 1 : (F32 ? 8 : 6));
+    default: return set != FX_AUTO ? set : (g->nitem_cell <= few ? 1 : (F32 ? 8 : 4));
     }
 }
 }  // namespace
