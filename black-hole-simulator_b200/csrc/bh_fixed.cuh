@@ -89,7 +89,8 @@ __device__ inline void atomic_max_pos(double* slot, double v) {
 // ======================================================================
 // the item loop.  Without a queue, CTA t takes item t of the launch's work
 // list.  With one (the persistent form: a grid of resident CTAs), each CTA
-// takes items from a device counter until none is left; the last CTA to
+// starts with item blockIdx and takes further ones from a device counter until
+// none is left; the last CTA to
 // finish resets the counter for the next launch of the slot, so a step
 // needs no extra launch or memset and records into a CUDA graph as is.
 // ======================================================================
@@ -107,14 +108,17 @@ __device__ __forceinline__ void for_items(const Queue& q, Body body) {
         body((int)blockIdx.x);
         return;
     }
-    __shared__ int s_item;
-    for (;;) {
-        if (threadIdx.x == 0) s_item = atomicAdd(q.head, 1);
-        __syncthreads();
-        const int t = s_item;
-        __syncthreads();
-        if (t >= q.nitem) break;
+    // the first item is the CTA's own index; the next one's fetch is issued
+    // ahead of the current item's work, so its round trip is hidden
+    __shared__ int s_item[2];
+    int t = blockIdx.x;
+    for (int p = 0; t < q.nitem; p ^= 1) {
+        int next = 0;
+        if (threadIdx.x == 0) next = (int)gridDim.x + atomicAdd(q.head, 1);
         body(t);
+        if (threadIdx.x == 0) s_item[p] = next;
+        __syncthreads();
+        t = s_item[p];
     }
     if (threadIdx.x == 0) {
         __threadfence();
