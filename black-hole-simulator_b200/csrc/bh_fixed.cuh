@@ -315,8 +315,9 @@ __device__ inline int shell_decode(int n, int g, int e, int& i, int& j, int& k) 
         return 1;
     }
     e -= s2;
-    if (e < s3) {   // i, j in [0,n), k in the ghost planes
-        int q = e / (n * n), r = e % (n * n);
+    if (e < s3) {   // i, j in [0,n), k in the ghost planes (fastest: a row's
+                    // ghosts share its sectors)
+        int q = e % h, r = e / h;
         i = r / n; j = r % n;
         k = q < g ? q - g : n + q - g;
         return 1;
@@ -361,97 +362,136 @@ __device__ inline double mm_slope(double a, double b, double c) {   // minmod of
     if (l * r <= 0.0) return 0.0;
     return fabs(l) < fabs(r) ? l : r;
 }
+// the source block of a ghost: its box and what its cells are to a block of
+// n^3 cells (0 copy, 1 restriction, 2 prolongation)
+struct GhostSrc {
+    int n, kind;
+    int64_t off;
+};
+__device__ inline GhostSrc ghost_block(const Grid& G, int s, int n) {
+    const bh_fx_block* S = G.blk + s;
+    return GhostSrc{S->n, S->n == n ? 0 : (S->n > n ? 1 : 2), S->off};
+}
+// (a box has fewer than 2^31 entries)
+__device__ inline int64_t bidx(const GhostSrc& b, int i, int j, int k) {
+    const int S = b.n + 2 * FX_GB + 1;
+    return b.off + (((i + FX_GB) * S + (j + FX_GB)) * S + (k + FX_GB));
+}
 template <typename WT>
-__global__ void __launch_bounds__(FX_TPB) k_fx_ghost(Grid G, const int32_t* items, int stage, int pass, Queue Q) {
-    for_items(Q, [&](int t) FX_INLINE {
-        const int32_t b = items[2 * t];
-        const bh_fx_block B = G.blk[b];
-        if (pass > 0 && B.level != pass) return;
-        const int n = B.n;
-        const int e = items[2 * t + 1] + threadIdx.x;
-        int i, j, k;
-        if (!shell_decode(n, G.gdepth, e, i, j, k)) return;
-        const int64_t N = G.ncell;
-        WT* W = (WT*)G.W;
-        double* Bf = stage ? G.Bf1 : G.Bf;
-        const int64_t c = bidx(B, i, j, k);
-        {
-            int si = i, sj = j, sk = k;
-            int s = ghost_source(G, b, n, -1, si, sj, sk);
-            const bh_fx_block S = G.blk[s];
-            const int kind = S.n == n ? 0 : (S.n > n ? 1 : 2);   // copy, restrict, prolong
-            if ((kind == 2) == (pass > 0)) {
-                if (kind == 0) {
-                    const int64_t sc = bidx(S, si, sj, sk);
-                    for (int v = 0; v < 8; v++) W[v * N + c] = W[v * N + sc];
-                } else if (kind == 1) {
-                    for (int v = 0; v < 8; v++) {
-                        double sum = 0.0;
-                        for (int a = 0; a < 2; a++)
-                            for (int q = 0; q < 2; q++)
-                                for (int r = 0; r < 2; r++)
-                                    sum += (double)W[v * N + bidx(S, 2 * si + a, 2 * sj + q, 2 * sk + r)];
-                        W[v * N + c] = (WT)(0.125 * sum);
-                    }
-                } else {
-                    const int ic = si >> 1, jc = sj >> 1, kc = sk >> 1;
-                    const double gx = (si & 1) ? 0.25 : -0.25, gy = (sj & 1) ? 0.25 : -0.25, gz = (sk & 1) ? 0.25 : -0.25;
-                    for (int v = 0; v < 8; v++) {
-                        const WT* Wv = W + v * N;
-                        double w0 = (double)Wv[bidx(S, ic, jc, kc)];
-                        double sx = mm_slope((double)Wv[bidx(S, ic - 1, jc, kc)], w0, (double)Wv[bidx(S, ic + 1, jc, kc)]);
-                        double sy = mm_slope((double)Wv[bidx(S, ic, jc - 1, kc)], w0, (double)Wv[bidx(S, ic, jc + 1, kc)]);
-                        double sz = mm_slope((double)Wv[bidx(S, ic, jc, kc - 1)], w0, (double)Wv[bidx(S, ic, jc, kc + 1)]);
-                        W[v * N + c] = (WT)(w0 + gx * sx + gy * sy + gz * sz);
-                    }
-                }
-            }
-        }
-        // the lower faces of this ghost cell that the flux kernel reads: normal
-        // index 0..n, transverse index -1..n, outside the block's own faces
-        // (transverse 0..n-1)
-        for (int d = 0; d < 3; d++) {
-            int cc[3] = {i, j, k};
-            if (cc[d] < 0 || cc[d] > n) continue;
-            bool need = true;
-            for (int q = 0; q < 3; q++)
-                if (q != d && (cc[q] < -1 || cc[q] > n)) need = false;
-            if (!need) continue;
-            int t[3] = {i, j, k};
-            int s = ghost_source(G, b, n, d, t[0], t[1], t[2]);
-            const bh_fx_block S = G.blk[s];
-            const int kind = S.n == n ? 0 : (S.n > n ? 1 : 2);
-            if ((kind == 2) != (pass > 0)) continue;
-            const double* Bd = Bf + d * N;
-            double v;
+__global__ void __launch_bounds__(FX_TPB, 8) k_fx_ghost(Grid G, const int32_t* items, int stage, int pass) {
+    const int t = blockIdx.x;
+    const int32_t b = items[2 * t];
+    const bh_fx_block B = G.blk[b];
+    if (pass > 0 && B.level != pass) return;
+    const int n = B.n;
+    const int e = items[2 * t + 1] + threadIdx.x;
+    int i, j, k;
+    if (!shell_decode(n, G.gdepth, e, i, j, k)) return;
+    const int64_t N = G.ncell;
+    WT* W = (WT*)G.W;
+    double* Bf = stage ? G.Bf1 : G.Bf;
+    const int64_t c = bidx(B, i, j, k);
+    // Bound: memory latency and sectors (the shell's rows are short, its
+    // k-ghosts single cells): values are loaded before the first is stored (a
+    // load behind a store that may alias it waits for it), the source block is
+    // looked up once for a cell and its faces, and a row's k-ghosts are
+    // neighbouring lanes.  With one CTA per item: blocks of three levels 174 ->
+    // 135 us mixed, 215 -> 172 FP64, 96^3 in 32^3 blocks 42 -> 22 FP64.
+    WT val[8];
+    int si = i, sj = j, sk = k;
+    const GhostSrc S = ghost_block(G, ghost_source(G, b, n, -1, si, sj, sk), n);
+    const bool have = (S.kind == 2) == (pass > 0);
+    {
+        if (have) {
+            const int kind = S.kind;
             if (kind == 0) {
-                v = Bd[bidx(S, t[0], t[1], t[2])];
+                const int64_t sc = bidx(S, si, sj, sk);
+#pragma unroll
+                for (int v = 0; v < 8; v++) val[v] = W[v * N + sc];
             } else if (kind == 1) {
-                // the 4 fine faces on this coarse face
-                int f[3] = {2 * t[0], 2 * t[1], 2 * t[2]};
-                const int t1 = (d + 1) % 3, t2 = (d + 2) % 3;
-                double sum = 0.0;
-                for (int a = 0; a < 2; a++)
-                    for (int q = 0; q < 2; q++) {
-                        int g[3] = {f[0], f[1], f[2]};
-                        g[t1] += a;
-                        g[t2] += q;
-                        sum += Bd[bidx(S, g[0], g[1], g[2])];
-                    }
-                v = 0.25 * sum;
+#pragma unroll
+                for (int v = 0; v < 8; v++) {
+                    double sum = 0.0;
+                    for (int a = 0; a < 2; a++)
+                        for (int q = 0; q < 2; q++)
+                            for (int r = 0; r < 2; r++)
+                                sum += (double)W[v * N + bidx(S, 2 * si + a, 2 * sj + q, 2 * sk + r)];
+                    val[v] = (WT)(0.125 * sum);
+                }
             } else {
-                int g[3] = {t[0] >> 1, t[1] >> 1, t[2] >> 1};
-                if (t[d] & 1) {   // between two coarse faces
-                    int h[3] = {g[0], g[1], g[2]};
-                    h[d] += 1;
-                    v = 0.5 * (Bd[bidx(S, g[0], g[1], g[2])] + Bd[bidx(S, h[0], h[1], h[2])]);
-                } else {
-                    v = Bd[bidx(S, g[0], g[1], g[2])];
+                const int ic = si >> 1, jc = sj >> 1, kc = sk >> 1;
+                const double gx = (si & 1) ? 0.25 : -0.25, gy = (sj & 1) ? 0.25 : -0.25, gz = (sk & 1) ? 0.25 : -0.25;
+#pragma unroll
+                for (int v = 0; v < 8; v++) {
+                    const WT* Wv = W + v * N;
+                    double w0 = (double)Wv[bidx(S, ic, jc, kc)];
+                    double sx = mm_slope((double)Wv[bidx(S, ic - 1, jc, kc)], w0, (double)Wv[bidx(S, ic + 1, jc, kc)]);
+                    double sy = mm_slope((double)Wv[bidx(S, ic, jc - 1, kc)], w0, (double)Wv[bidx(S, ic, jc + 1, kc)]);
+                    double sz = mm_slope((double)Wv[bidx(S, ic, jc, kc - 1)], w0, (double)Wv[bidx(S, ic, jc, kc + 1)]);
+                    val[v] = (WT)(w0 + gx * sx + gy * sy + gz * sz);
                 }
             }
-            Bf[d * N + c] = v;
         }
-    });
+    }
+    // the lower faces of this ghost cell that the flux kernel reads: normal
+    // index 0..n, transverse index -1..n, outside the block's own faces
+    // (transverse 0..n-1)
+    double face[3];
+    bool fill[3] = {false, false, false};
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        int cc[3] = {i, j, k};
+        if (cc[d] < 0 || cc[d] > n) continue;
+        bool need = true;
+        for (int q = 0; q < 3; q++)
+            if (q != d && (cc[q] < -1 || cc[q] > n)) need = false;
+        if (!need) continue;
+        // a face lies with its cell, but for the one at the block's upper
+        // end (normal index n), which is the block's own in that direction
+        int t[3] = {si, sj, sk};
+        GhostSrc T = S;
+        if (cc[d] == n) {
+            t[0] = i; t[1] = j; t[2] = k;
+            T = ghost_block(G, ghost_source(G, b, n, d, t[0], t[1], t[2]), n);
+        }
+        const int kind = T.kind;
+        if ((kind == 2) != (pass > 0)) continue;
+        const double* Bd = Bf + d * N;
+        double v;
+        if (kind == 0) {
+            v = Bd[bidx(T, t[0], t[1], t[2])];
+        } else if (kind == 1) {
+            // the 4 fine faces on this coarse face
+            int f[3] = {2 * t[0], 2 * t[1], 2 * t[2]};
+            const int t1 = (d + 1) % 3, t2 = (d + 2) % 3;
+            double sum = 0.0;
+            for (int a = 0; a < 2; a++)
+                for (int q = 0; q < 2; q++) {
+                    int g[3] = {f[0], f[1], f[2]};
+                    g[t1] += a;
+                    g[t2] += q;
+                    sum += Bd[bidx(T, g[0], g[1], g[2])];
+                }
+            v = 0.25 * sum;
+        } else {
+            int g[3] = {t[0] >> 1, t[1] >> 1, t[2] >> 1};
+            if (t[d] & 1) {   // between two coarse faces
+                int h[3] = {g[0], g[1], g[2]};
+                h[d] += 1;
+                v = 0.5 * (Bd[bidx(T, g[0], g[1], g[2])] + Bd[bidx(T, h[0], h[1], h[2])]);
+            } else {
+                v = Bd[bidx(T, g[0], g[1], g[2])];
+            }
+        }
+        face[d] = v;
+        fill[d] = true;
+    }
+    if (have)
+#pragma unroll
+        for (int v = 0; v < 8; v++) W[v * N + c] = val[v];
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+        if (fill[d]) Bf[d * N + c] = face[d];
 }
 
 // ======================================================================
@@ -718,45 +758,44 @@ __global__ void __launch_bounds__(FX_TPB) k_fx_emf(Grid G, const int32_t* items,
 // so every copy of a shared face sees the same circulation and the face
 // field of the coarse side stays the mean of the fine faces (div B at
 // roundoff).  Levels differ by one at most, so one pass suffices.
-__global__ void __launch_bounds__(FX_TPB) k_fx_emf_fix(Grid G, const int32_t* items, Queue Q) {
-    for_items(Q, [&](int t) FX_INLINE {
-        const int32_t b = items[2 * t];
-        const bh_fx_block B = G.blk[b];
-        const int n = B.n, m = n + 2;
-        const int e = items[2 * t + 1] + threadIdx.x;
-        if (e >= m * m * m) return;
-        const int p[3] = {e / (m * m) - 1, (e / m) % m - 1, e % m - 1};
-        if (p[0] < 0 || p[1] < 0 || p[2] < 0) return;
-        const int64_t N = G.ncell;
-        const int32_t* nb = G.nbr + (int64_t)b * 27;
-        for (int d = 0; d < 3; d++) {          // edge direction
-            if (p[d] >= n) continue;
-            const int t1 = (d + 1) % 3, t2 = (d + 2) % 3;
-            const int o1 = p[t1] == 0 ? -1 : (p[t1] == n ? 1 : 0);
-            const int o2 = p[t2] == 0 ? -1 : (p[t2] == n ? 1 : 0);
-            if (o1 == 0 && o2 == 0) continue;  // not on the boundary
-            // the cubes sharing the edge: offsets (a1 o1, a2 o2), (a1, a2) != (0, 0)
-            for (int a1 = 0; a1 <= (o1 != 0); a1++)
-                for (int a2 = 0; a2 <= (o2 != 0); a2++) {
-                    if (!a1 && !a2) continue;
-                    int o[3] = {0, 0, 0};
-                    o[t1] = a1 * o1;
-                    o[t2] = a2 * o2;
-                    const int s = nb[(o[0] + 1) * 9 + (o[1] + 1) * 3 + (o[2] + 1)];
-                    if (s < 0) continue;
-                    const bh_fx_block S = G.blk[s];
-                    if (S.n != 2 * n) continue;
-                    // the two fine edges along this one, in the finer block's frame
-                    int f[3] = {2 * (p[0] - o[0] * n), 2 * (p[1] - o[1] * n), 2 * (p[2] - o[2] * n)};
-                    int g[3] = {f[0], f[1], f[2]};
-                    g[d] += 1;
-                    const double* Es = G.E + d * N;
-                    G.E[d * N + bidx(B, p[0], p[1], p[2])] = 0.5 * (Es[bidx(S, f[0], f[1], f[2])] + Es[bidx(S, g[0], g[1], g[2])]);
-                    a1 = 2;   // done with this edge
-                    break;
-                }
-        }
-    });
+__global__ void __launch_bounds__(FX_TPB) k_fx_emf_fix(Grid G, const int32_t* items) {
+    const int t = blockIdx.x;
+    const int32_t b = items[2 * t];
+    const bh_fx_block B = G.blk[b];
+    const int n = B.n, m = n + 2;
+    const int e = items[2 * t + 1] + threadIdx.x;
+    if (e >= m * m * m) return;
+    const int p[3] = {e / (m * m) - 1, (e / m) % m - 1, e % m - 1};
+    if (p[0] < 0 || p[1] < 0 || p[2] < 0) return;
+    const int64_t N = G.ncell;
+    const int32_t* nb = G.nbr + (int64_t)b * 27;
+    for (int d = 0; d < 3; d++) {          // edge direction
+        if (p[d] >= n) continue;
+        const int t1 = (d + 1) % 3, t2 = (d + 2) % 3;
+        const int o1 = p[t1] == 0 ? -1 : (p[t1] == n ? 1 : 0);
+        const int o2 = p[t2] == 0 ? -1 : (p[t2] == n ? 1 : 0);
+        if (o1 == 0 && o2 == 0) continue;  // not on the boundary
+        // the cubes sharing the edge: offsets (a1 o1, a2 o2), (a1, a2) != (0, 0)
+        for (int a1 = 0; a1 <= (o1 != 0); a1++)
+            for (int a2 = 0; a2 <= (o2 != 0); a2++) {
+                if (!a1 && !a2) continue;
+                int o[3] = {0, 0, 0};
+                o[t1] = a1 * o1;
+                o[t2] = a2 * o2;
+                const int s = nb[(o[0] + 1) * 9 + (o[1] + 1) * 3 + (o[2] + 1)];
+                if (s < 0) continue;
+                const bh_fx_block S = G.blk[s];
+                if (S.n != 2 * n) continue;
+                // the two fine edges along this one, in the finer block's frame
+                int f[3] = {2 * (p[0] - o[0] * n), 2 * (p[1] - o[1] * n), 2 * (p[2] - o[2] * n)};
+                int g[3] = {f[0], f[1], f[2]};
+                g[d] += 1;
+                const double* Es = G.E + d * N;
+                G.E[d * N + bidx(B, p[0], p[1], p[2])] = 0.5 * (Es[bidx(S, f[0], f[1], f[2])] + Es[bidx(S, g[0], g[1], g[2])]);
+                a1 = 2;   // done with this edge
+                break;
+            }
+    }
 }
 
 // PART 3: the whole update; 1: the conserved state (source, divergence,
@@ -1295,9 +1334,12 @@ int fx_prims(const bh_fx_params* P, const bh_fx_grid* g, int32_t stage, int32_t 
 }
 int fx_ghost_pass(const bh_fx_params*, const bh_fx_grid* g, int32_t stage, int32_t pass, void* s) {
     fx::Grid G = fx::grid_of(g);
+    // one CTA per item, with or without a queue: an item is a few round trips
+    // to memory, of very different lengths, and a persistent CTA's barrier
+    // between items makes its warps wait for the longest (three levels, FP64,
+    // passes 0-2: 126 + 44 + 28 us persistent, 107 + 37 + 21 like this)
     if (g->nitem_ghost)
-        fx::k_fx_ghost<FRT><<<fx_grid((const void*)fx::k_fx_ghost<FRT>, g->nitem_ghost, g), fx::FX_TPB, 0, fxs(s)>>>(
-            G, g->items_ghost, stage, pass, fx_q(g, QS_GHOST, g->nitem_ghost));
+        fx::k_fx_ghost<FRT><<<g->nitem_ghost, fx::FX_TPB, 0, fxs(s)>>>(G, g->items_ghost, stage, pass);
     return fx_launched();
 }
 int fx_ghosts(const bh_fx_params* P, const bh_fx_grid* g, int32_t stage, void* s) {
@@ -1329,9 +1371,8 @@ int fx_update_parts(const bh_fx_params* P, const bh_fx_grid* g, int32_t stage, i
         fx::k_fx_emf<FRT><<<fx_grid((const void*)fx::k_fx_emf<FRT>, g->nitem_pos, g), fx::FX_TPB, 0, fxs(s)>>>(
             G, g->items_pos, fx_q(g, QS_EMF, g->nitem_pos));
     if (!(parts & 2)) return fx_launched();
-    if (g->E && g->nitem_pos && g->maxlevel > 0)
-        fx::k_fx_emf_fix<<<fx_grid((const void*)fx::k_fx_emf_fix, g->nitem_pos, g), fx::FX_TPB, 0, fxs(s)>>>(
-            G, g->items_pos, fx_q(g, QS_EMF_FIX, g->nitem_pos));
+    if (g->E && g->nitem_pos && g->maxlevel > 0)   // (one CTA per item, as the ghost fill: most items have no work)
+        fx::k_fx_emf_fix<<<g->nitem_pos, fx::FX_TPB, 0, fxs(s)>>>(G, g->items_pos);
     if (g->nitem_cell && fx_choose(BH_FX_TUNE_SPLIT, P, g)) {
 #define L_(M) fx::k_fx_update<FRT, FRT, FRT, M, 1><<<fx_grid((const void*)fx::k_fx_update<FRT, FRT, FRT, M, 1>, g->nitem_cell, g), fx::FX_TPB, 0, fxs(s)>>>(p, G, g->items_cell, stage, P->cfl, fx_q(g, QS_UPDATE, g->nitem_cell))
         FX_TUNED(fx_choose(BH_FX_TUNE_UPDATE, P, g), L_)
