@@ -56,6 +56,8 @@ inline FxPar par_of(const bh_fx_params* p) {
     q.gf = (p->gamma - 1.0) / p->gamma;
     q.v2max = 1.0 - 1.0 / (p->W_max * p->W_max);
     q.flags = p->flags;
+    auto in = [](double v) { return v == 0.0 || (v >= 1e-30 && v <= 1e30); };
+    q.sane = in(fabs(p->M)) && in(fabs(p->a)) && p->gamma >= 1.001 && p->gamma <= 100.0;
     return q;
 }
 
@@ -502,10 +504,10 @@ __global__ void __launch_bounds__(FX_TPB, 8) k_fx_ghost(Grid G, const int32_t* i
 // ======================================================================
 // the face computation; sten(v, o) is variable v of the cell o = -2..1
 // (PLM) or -3..2 (PPM, where PPM6) steps along d from (i, j, k) (the face
-// lies between o = -1 and o = 0)
+// lies between o = -1 and o = 0); the same value is sp[v vs + o os]
 template <typename RT, typename FT, bool PPM6, typename Sten>
 __device__ __forceinline__ void face_flux_at(const FxPar& P, const Grid& G, const bh_fx_block& B, int i, int j, int k,
-                                             int d, const double* Bfs, const Sten& sten) {
+                                             int d, const double* Bfs, const Sten& sten, const RT* sp, int64_t vs, int os) {
     const int64_t N = G.ncell;
     const int64_t c = bidx(B, i, j, k);
     KSm<RT> m;
@@ -528,11 +530,6 @@ __device__ __forceinline__ void face_flux_at(const FxPar& P, const Grid& G, cons
             ks_metric(P, x[0], x[1], x[2], mk);
             ks_cast(mk, m);
         }
-    } else {
-        double x[3];
-        cell_centre(B, i, j, k, x);
-        x[d] -= 0.5 * B.dx;
-        face_geometry<RT>(P, x, m);
     }
     RT wL[8], wR[8];
 #pragma unroll   // (wL, wR stay in registers only if every index is a constant)
@@ -547,11 +544,18 @@ __device__ __forceinline__ void face_flux_at(const FxPar& P, const Grid& G, cons
     }
     // (the limiters keep every face value between its two cells' values, so
     // face densities and pressures stay positive)
-    RT Bn = RT(Bfs[d * N + c]) * m.alpha;   // alpha = 1 / sqrt(gamma)
-    wL[P_B + d] = Bn;
-    wR[P_B + d] = Bn;
     RT F[8];
-    hll_face(m, RT(P.gamma), RT(P.gg), d, wL, wR, F);
+    if constexpr (sizeof(RT) == sizeof(double)) {
+        double x[3];
+        cell_centre(B, i, j, k, x);
+        x[d] -= 0.5 * B.dx;
+        face64(P, x, d, Bfs[d * N + c], wL, wR, sp, vs, os, F);
+    } else {
+        RT Bn = RT(Bfs[d * N + c]) * m.alpha;   // alpha = 1 / sqrt(gamma)
+        wL[P_B + d] = Bn;
+        wR[P_B + d] = Bn;
+        hll_face(m, RT(P.gamma), RT(P.gg), d, wL, wR, F);
+    }
     FT* Fo = (FT*)G.F;
     for (int v = 0; v < 8; v++) Fo[((int64_t)d * 8 + v) * N + c] = (FT)F[v];
 }
@@ -563,7 +567,7 @@ __device__ inline void face_flux(const FxPar& P, const Grid& G, const bh_fx_bloc
     const int64_t N = G.ncell;
     const WT* Wc = (const WT*)G.W + bidx(B, i, j, k);
     const int st = d == 0 ? bstride_i(B) : (d == 1 ? bstride_j(B) : 1);
-    face_flux_at<RT, FT, true>(P, G, B, i, j, k, d, Bfs, [&](int v, int o) { return RT(Wc[v * N + o * st]); });
+    face_flux_at<RT, FT, true>(P, G, B, i, j, k, d, Bfs, [&](int v, int o) { return RT(Wc[v * N + o * st]); }, Wc, N, st);
 }
 
 template <typename RT, typename WT, typename FT, int MINB>
@@ -666,12 +670,14 @@ __global__ void __launch_bounds__(FX_TPB, MINB) k_fx_flux_tile(FxPar P, Grid G, 
         // (PLM only: the launch keeps PPM's wider stencil on k_fx_flux)
         if (i >= 0)
             face_flux_at<RT, FT, false>(P, G, B, i, j, k, 0, Bfs,
-                                        [&](int v, int s) { return RT(sW[v][o + s * (FX_HJ * FX_HKP)]); });
+                                        [&](int v, int s) { return RT(sW[v][o + s * (FX_HJ * FX_HKP)]); }, &sW[0][o],
+                                        FX_HBOX, FX_HJ * FX_HKP);
         if (j >= 0)
             face_flux_at<RT, FT, false>(P, G, B, i, j, k, 1, Bfs,
-                                        [&](int v, int s) { return RT(sW[v][o + s * FX_HKP]); });
+                                        [&](int v, int s) { return RT(sW[v][o + s * FX_HKP]); }, &sW[0][o], FX_HBOX, FX_HKP);
         if (k >= 0)
-            face_flux_at<RT, FT, false>(P, G, B, i, j, k, 2, Bfs, [&](int v, int s) { return RT(sW[v][o + s]); });
+            face_flux_at<RT, FT, false>(P, G, B, i, j, k, 2, Bfs, [&](int v, int s) { return RT(sW[v][o + s]); },
+                                        &sW[0][o], FX_HBOX, 1);
     });
 }
 
@@ -1275,10 +1281,10 @@ namespace {
 //   con2prim  7 (mixed), 6: 128^3 237 -> 122 / 337 -> 197, lev 175 -> 105 / 241 -> 149.
 //   fluxes    the stencil staged where the tiles pad the positions by at most
 //             a tenth (blocks of ~100^3 on): 128^3 (8 %) 275 against 292 /
-//             587 against 621 unstaged, 64^3 (16 %) 45 against 42 / 94 against 87.
+//             542 against 562 unstaged, 64^3 (16 %) 45 against 42 / 94 against 87.
 //             Resident CTAs 8 in FP32 (128^3 365 -> 275, PPM 540 -> 431);
-//             in FP64 4 staged (697 -> 587) and 5 unstaged (782 -> 621, PPM
-//             1082 -> 856, lev 812 -> 636): more would spill.
+//             in FP64 4 staged (697 -> 542) and 5 unstaged (782 -> 562, PPM
+//             1082 -> 801): more would spill.
 //   update    8 in FP32, 4 in FP64 (whose early loads fill the registers); as
 //             its two kernels with edge EMFs in arrays (lev 249 -> 210 / 249 ->
 //             248) and on grids of 8192 items, in FP64 2048, or more (128^3

@@ -42,6 +42,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <math.h>
+#include "bh_div.cuh"
 
 #ifndef BH_HD
 #define BH_HD __host__ __device__
@@ -71,6 +72,7 @@ struct FxPar {
     // derived once per launch: Gamma/(Gamma-1), (Gamma-1)/Gamma, the v^2 of W_max
     double gg, gf, v2max;
     int flags;                // BH_FX_C2P_FP64
+    int sane;                 // M, a and gamma within the range of Ops<double, true>
 };
 
 template <typename T>
@@ -81,6 +83,42 @@ template <typename T>
 BH_FI T fabs_(T a) { return a < T(0) ? -a : a; }
 BH_FI double sqrt_(double x) { return sqrt(x); }
 BH_FI float sqrt_(float x) { return sqrtf(x); }
+
+// ----------------------------------------------------------------------
+// the divisions and square roots of the face work.  FAST (double only): the
+// branch-free ones of bh_div.cuh, with `ok` cleared where an operand may
+// leave their range (the caller then takes the plain form); the same bits.
+// ----------------------------------------------------------------------
+template <typename T, bool FAST>
+struct Ops {
+    static BH_FI void need(bool&, bool) {}
+    static BH_FI T recip(T b) { return T(1) / b; }
+    static BH_FI T quot(T a, T b) { return a / b; }
+    static BH_FI T quot_by(T a, T b, T) { return a / b; }
+    static BH_FI T quot_near(T a, T b, T) { return a / b; }
+    static BH_FI T root(T x, T& inv) { T s = sqrt_(x); inv = T(1) / s; return s; }
+    static BH_FI T root0(T x, bool&) { return sqrt_(x); }
+};
+template <>
+struct Ops<double, true> {
+    static BH_FI void need(bool& ok, bool c) { ok = ok && c; }
+    static BH_FI double recip(double b) { return bh::rcp_any(b); }
+    static BH_FI double quot(double a, double b) { return bh::div_by(a, b, bh::rcp_any(b)); }
+    static BH_FI double quot_by(double a, double b, double y) { return bh::div_by(a, b, y); }   // y = 1 / b
+    static BH_FI double quot_near(double a, double b, double y) {                               // y near 1 / b
+        return bh::div_by(a, b, bh::rcp_polish_any(b, y));
+    }
+    static BH_FI double root(double x, double& inv) {
+        double i2, s = bh::sqrt_rn(x, i2);
+        inv = bh::rcp_polish_any(s, 2.0 * i2);
+        return s;
+    }
+    static BH_FI double root0(double x, bool& ok) {   // x >= 0
+        double i2, s = bh::sqrt_rn(x, i2);
+        need(ok, x == 0.0 || x >= 1e-100);
+        return x > 0.0 ? s : 0.0;
+    }
+};
 
 // ======================================================================
 // metric
@@ -110,24 +148,25 @@ BH_FI int sym(int i, int j) {   // index into the 6-entry symmetric storage
     return a == 0 ? b : (a == 1 ? 2 + b : 5);
 }
 
-template <typename T>
-BH_FI void ks_metric(const FxPar& P, T x, T y, T z, KSb<T>& m) {
+template <typename T, bool FAST>
+BH_FI void ks_metric_ops(const FxPar& P, T x, T y, T z, KSb<T>& m, bool& ok) {
+    using O = Ops<T, FAST>;
     const T a = T(P.a), a2 = a * a;
     T r2 = ks_r2(a, x, y, z);
-    T r = sqrt_(r2);
+    O::need(ok, P.sane && r2 >= T(1e-60) && r2 <= T(1e60) && (z == T(0) || fabs_(z) >= T(1e-60)));
+    T ir, r = O::root(r2, ir);
     T q = r2 * r2 + a2 * z * z;
     // on the disc z = 0, x^2 + y^2 <= a^2 (r = 0) the metric is flat
-    T H = q > T(0) ? T(P.M) * r * r2 / q : T(0);
-    T ir2a = T(1) / (r2 + a2);
+    T H = q > T(0) ? O::quot(T(P.M) * r * r2, q) : T(0);
+    T ir2a = O::recip(r2 + a2);
     m.r = r;
     m.H = H;
     m.l[0] = (r * x + a * y) * ir2a;
     m.l[1] = (r * y - a * x) * ir2a;
-    m.l[2] = r > T(0) ? z / r : T(0);
+    m.l[2] = r > T(0) ? O::quot_by(z, r, ir) : T(0);
     T h2 = T(2) * H, f = T(1) + h2;
-    m.sqrtgam = sqrt_(f);
-    m.alpha = T(1) / m.sqrtgam;
-    T hf = h2 / f;
+    m.sqrtgam = O::root(f, m.alpha);
+    T hf = O::quot_near(h2, f, m.alpha * m.alpha);
     for (int i = 0; i < 3; i++) m.beta[i] = hf * m.l[i];
     for (int i = 0; i < 3; i++)
         for (int j = i; j < 3; j++) {
@@ -135,6 +174,12 @@ BH_FI void ks_metric(const FxPar& P, T x, T y, T z, KSb<T>& m) {
             m.g[sym(i, j)] = (i == j ? T(1) : T(0)) + h2 * ll;
             m.gi[sym(i, j)] = (i == j ? T(1) : T(0)) - hf * ll;
         }
+}
+
+template <typename T>
+BH_FI void ks_metric(const FxPar& P, T x, T y, T z, KSb<T>& m) {
+    bool ok = true;
+    ks_metric_ops<T, false>(P, x, y, z, m, ok);
 }
 
 // first derivatives: dH[k] = d_k H, dl[k][i] = d_k l_i (d_k l_0 = 0)
@@ -194,17 +239,19 @@ struct Derived {
     RT W, iW, rhoh, v[3], vl[3], Bl[3], B2, Bv, b2, rhohW2, ptot;
     RT u2, ggp;   // W^2 - 1 = u_i u^i, and Gamma/(Gamma-1) p
 };
-template <typename RT>
 // gg = Gamma / (Gamma - 1)
-BH_FI void derive(const KSm<RT>& m, RT gg, const RT* w, Derived<RT>& d) {
+template <typename RT, bool FAST>
+BH_FI void derive_ops(const KSm<RT>& m, RT gg, const RT* w, Derived<RT>& d, bool& ok) {
+    using O = Ops<RT, FAST>;
     RT ut[3] = {w[P_UT], w[P_UT + 1], w[P_UT + 2]};
     RT B[3] = {w[P_B], w[P_B + 1], w[P_B + 2]};
     RT utl[3];
     lower(m.g, ut, utl);
     RT u2 = utl[0] * ut[0] + utl[1] * ut[1] + utl[2] * ut[2];
     d.u2 = u2;
-    d.W = sqrt_(RT(1) + u2);
-    RT iW = RT(1) / d.W;
+    O::need(ok, u2 >= RT(0) && u2 <= RT(1e12));
+    RT iW;
+    d.W = O::root(RT(1) + u2, iW);
     d.iW = iW;
     for (int i = 0; i < 3; i++) { d.v[i] = ut[i] * iW; d.vl[i] = utl[i] * iW; }
     lower(m.g, B, d.Bl);
@@ -216,6 +263,11 @@ BH_FI void derive(const KSm<RT>& m, RT gg, const RT* w, Derived<RT>& d) {
     d.rhoh = rhoh;
     d.rhohW2 = rhoh * d.W * d.W;
     d.ptot = w[P_PRS] + RT(0.5) * d.b2;
+}
+template <typename RT>
+BH_FI void derive(const KSm<RT>& m, RT gg, const RT* w, Derived<RT>& d) {
+    bool ok = true;
+    derive_ops<RT, false>(m, gg, w, d, ok);
 }
 // densitised conserved state of primitives w (B slots: sqrt(gamma) B)
 template <typename RT>
@@ -263,22 +315,29 @@ BH_FI void phys_flux(const KSm<RT>& m, int dd, const RT* w, const Derived<RT>& d
 }
 
 // fast magnetosonic signal speeds lambda-, lambda+ in direction dd
-template <typename RT>
-BH_FI void signal_speeds(const KSm<RT>& m, RT gamma, int dd, const RT* w, const Derived<RT>& d, RT& lm,
-                                RT& lp) {
+template <typename RT, bool FAST>
+BH_FI void signal_speeds_ops(const KSm<RT>& m, RT gamma, int dd, const RT* w, const Derived<RT>& d, RT& lm, RT& lp,
+                             bool& ok) {
+    using O = Ops<RT, FAST>;
     RT rhoh = d.rhoh;
     // c_s^2 + v_A^2 - c_s^2 v_A^2 with c_s^2 = Gamma p / (rho h), v_A^2 = b^2 / (rho h + b^2)
-    RT c2 = (gamma * w[P_PRS] + d.b2) / (rhoh + d.b2);
+    O::need(ok, d.b2 >= RT(0) && w[P_PRS] >= RT(1e-100) && rhoh + d.b2 <= RT(1e100) && rhoh >= RT(1e-100));
+    RT c2 = O::quot(gamma * w[P_PRS] + d.b2, rhoh + d.b2);
     c2 = fmin_(fmax_(c2, RT(0)), RT(1));
     RT v2 = RT(1) - d.iW * d.iW;
     RT vd = d.v[dd];
     RT gdd = m.gi[dd == 0 ? 0 : (dd == 1 ? 3 : 5)];
-    RT den = RT(1) / (RT(1) - v2 * c2);
+    RT den = O::recip(RT(1) - v2 * c2);
     RT disc = (RT(1) - v2) * (gdd * (RT(1) - v2 * c2) - vd * vd * (RT(1) - c2));
-    RT rt = sqrt_(fmax_(c2 * disc, RT(0)));
+    RT rt = O::root0(fmax_(c2 * disc, RT(0)), ok);
     RT base = vd * (RT(1) - c2);
     lm = m.alpha * (base - rt) * den - m.beta[dd];
     lp = m.alpha * (base + rt) * den - m.beta[dd];
+}
+template <typename RT>
+BH_FI void signal_speeds(const KSm<RT>& m, RT gamma, int dd, const RT* w, const Derived<RT>& d, RT& lm, RT& lp) {
+    bool ok = true;
+    signal_speeds_ops<RT, false>(m, gamma, dd, w, d, lm, lp, ok);
 }
 
 // ======================================================================
@@ -373,30 +432,88 @@ BH_FI void ppm_face(const RT* a, RT& L, RT& R) {
 // field comes from the face (wL[P_B+dd] = wR[P_B+dd]).  Returns the larger
 // signal speed magnitude.
 // ======================================================================
-template <typename RT>
-BH_FI RT hll_face(const KSm<RT>& m, RT gamma, RT gg, int dd, const RT* wL, const RT* wR, RT* F) {
+template <typename RT, bool FAST>
+BH_FI RT hll_face_ops(const KSm<RT>& m, RT gamma, RT gg, int dd, const RT* wL, const RT* wR, RT* F, bool& ok) {
+    using O = Ops<RT, FAST>;
     Derived<RT> dL, dR;
-    derive(m, gg, wL, dL);
-    derive(m, gg, wR, dR);
+    derive_ops<RT, FAST>(m, gg, wL, dL, ok);
+    derive_ops<RT, FAST>(m, gg, wR, dR, ok);
     RT uL[8], uR[8], FL[8], FR[8];
     prim2cons(m, gamma, wL, dL, uL);
     prim2cons(m, gamma, wR, dR, uR);
     phys_flux(m, dd, wL, dL, uL, FL);
     phys_flux(m, dd, wR, dR, uR, FR);
     RT lmL, lpL, lmR, lpR;
-    signal_speeds(m, gamma, dd, wL, dL, lmL, lpL);
-    signal_speeds(m, gamma, dd, wR, dR, lmR, lpR);
+    signal_speeds_ops<RT, FAST>(m, gamma, dd, wL, dL, lmL, lpL, ok);
+    signal_speeds_ops<RT, FAST>(m, gamma, dd, wR, dR, lmR, lpR, ok);
     RT sl = fmin_(fmin_(lmL, lmR), RT(0));
     RT sr = fmax_(fmax_(lpL, lpR), RT(0));
     RT ds = sr - sl;
     if (ds > RT(0)) {
-        RT ids = RT(1) / ds, ss = sr * sl;
+        O::need(ok, ds >= RT(1e-100) && ds <= RT(1e100));
+        RT ids = O::recip(ds), ss = sr * sl;
         for (int v = 0; v < 8; v++) F[v] = (sr * FL[v] - sl * FR[v] + ss * (uR[v] - uL[v])) * ids;
     } else {
         for (int v = 0; v < 8; v++) F[v] = RT(0.5) * (FL[v] + FR[v]);
     }
     F[C_B + dd] = RT(0);
     return fmax_(sr, -sl);
+}
+template <typename RT>
+BH_FI RT hll_face(const KSm<RT>& m, RT gamma, RT gg, int dd, const RT* wL, const RT* wR, RT* F) {
+    bool ok = true;
+    return hll_face_ops<RT, false>(m, gamma, gg, dd, wL, wR, F, ok);
+}
+// the FP64 flux through the face centred at x, normal d, from the face states
+// (their normal field from the densitised face value Bf); FAST: `ok` cleared
+// where an operand leaves the range of the branch-free operations
+template <bool FAST>
+BH_FI void face64_ops(const FxPar& P, const double* x, int d, double Bf, double* wL, double* wR, double* F, bool& ok) {
+    KS mk;
+    ks_metric_ops<double, FAST>(P, x[0], x[1], x[2], mk, ok);
+    KSm<double> m;
+    ks_cast(mk, m);
+    wL[P_B + d] = wR[P_B + d] = Bf * m.alpha;   // alpha = 1 / sqrt(gamma)
+    hll_face_ops<double, FAST>(m, P.gamma, P.gg, d, wL, wR, F, ok);
+}
+// the plain form from the stencil's cells in memory (variable v of the cell o
+// steps along d at p[v vs + o os]), out of line: hardly ever needed, it then
+// reconstructs anew, so that the face states need not outlive the fast form
+BH_HD inline __attribute__((noinline)) void face64_plain(double M, double a, double gamma, double gg, int limiter,
+                                                         const double* x, int d, double Bf, const double* p,
+                                                         int64_t vs, int os, double* F) {
+    FxPar P;
+    P.M = M; P.a = a; P.gamma = gamma; P.gg = gg; P.sane = 0;
+    double wL[8], wR[8];
+    for (int v = 0; v < 8; v++) {
+        const double* w = p + v * vs;
+        if (limiter == FX_PPM) {
+            const double c[6] = {w[-3 * os], w[-2 * os], w[-os], w[0], w[os], w[2 * os]};
+            ppm_face(c, wL[v], wR[v]);
+        } else {
+            plm_face(w[-2 * os], w[-os], w[0], w[os], limiter, wL[v], wR[v]);
+        }
+    }
+    bool ok = true;
+    face64_ops<false>(P, x, d, Bf, wL, wR, F, ok);
+}
+// Bound: the FP64 face work runs at half the FP64 pipe's rate, waiting on
+// chains of dependent operations at 16 to 20 warps per SM.  A face has 12
+// divisions and 7 square roots; the compiler's each end in a branch, so none
+// overlaps the next, and a reciprocal that is near at hand (1 / W from W's
+// square root, 1 / f from the lapse) is formed again.  128^3 PLM staged 586 ->
+// 542 us, unstaged 617 -> 562, PPM 855 -> 801; FMA 561 -> 509, 573 -> 515, 791 ->
+// 740; a 16^3 grid's launch 31 -> 26.  (In con2prim and the update the same
+// operations inlined cost more registers than they save: not used there.)
+BH_FI void face64(const FxPar& P, const double* x, int d, double Bf, double* wL, double* wR, const double* p,
+                  int64_t vs, int os, double* F) {
+    bool ok = true;
+    face64_ops<true>(P, x, d, Bf, wL, wR, F, ok);
+    if (!ok) {   // (copies: the arrays above stay in registers)
+        double f[8], c[3] = {x[0], x[1], x[2]};
+        face64_plain(P.M, P.a, P.gamma, P.gg, P.limiter, c, d, Bf, p, vs, os, f);
+        for (int v = 0; v < 8; v++) F[v] = f[v];
+    }
 }
 
 // ======================================================================
@@ -779,19 +896,6 @@ template <typename RT>
 BH_FI bool fp32_geometry(const double* x) {
     if (sizeof(RT) == sizeof(double)) return false;
     return x[0] * x[0] + x[1] * x[1] + x[2] * x[2] > FX_R_FP64 * FX_R_FP64;
-}
-// spatial metric at a face centre
-template <typename RT>
-BH_FI void face_geometry(const FxPar& P, const double* x, KSm<RT>& m) {
-    if (fp32_geometry<RT>(x)) {
-        KSb<float> mf;
-        ks_metric<float>(P, float(x[0]), float(x[1]), float(x[2]), mf);
-        ks_cast(mf, m);
-    } else {
-        KS mk;
-        ks_metric(P, x[0], x[1], x[2], mk);
-        ks_cast(mk, m);
-    }
 }
 // metric and derivatives at a cell centre, in RT
 template <typename RT>

@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "bhgpu.h"
+#include "bh_div.cuh"
 
 #ifndef BH_HD
 #define BH_HD __host__ __device__
@@ -330,58 +331,6 @@ using PtocOut = PtocOutT<double>;
 // ======================================================================
 // cons -> prim, conserved::ctop + f_df + cp_bd (physics/conserved.cpp:80-285)
 // ======================================================================
-// ---- correctly rounded division and square root without a branch --------
-// The compiler's FP64 division and square root end in a branch to a path for
-// extreme operands, so several of them run one after the other; in con2prim's
-// residual that chain is most of an iteration.  These round the same (to
-// nearest) for operands whose magnitudes and results stay within 2^+-500 (a
-// zero numerator too), which the caller checks for a whole expression at once:
-//   rcp_rn  a hardware approximation y0 (about 2^-20), one third-order step
-//           y = y0 (1 + e + e^2), e = 1 - b y0, then y + y (1 - b y): the
-//           nearest double to 1/b when y is within an ulp of it (Markstein
-//           1990, IBM J. Res. Dev. 34, 111);
-//   div_by  q = a y, then q + y (a - b q) with the remainder exact by FMA
-//           (same reference); one reciprocal serves several quotients;
-//   sqrt_rn Goldschmidt's iteration on g ~ sqrt(x), h ~ 1 / (2 sqrt(x)) from
-//           a hardware approximation, then g + h (x - g^2) (Markstein).
-// Markstein's step misses 1/b by an ulp where b's significand is all ones
-// (all_ones), which the caller checks too.  A host build takes the C operators.
-#ifdef __CUDA_ARCH__
-BH_HD inline bool all_ones(double b) { return ((__double2hiint(b) | (int)0xfff00000) & __double2loint(b)) == -1; }
-BH_HD inline double rcp_polish(double b, double y) { return fma(fma(-b, y, 1.0), y, y); }
-BH_HD inline double rcp_rn(double b) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    const double e = fma(-b, y, 1.0);
-    return rcp_polish(b, fma(fma(e, e, e), y, y));
-}
-// y: a reciprocal of b, correctly rounded
-BH_HD inline double div_by(double a, double b, double y) {
-    double q = a * y;
-    q = fma(fma(-b, q, a), y, q);
-    // (a zero quotient keeps its sign)
-    const int s = (__double2hiint(a) ^ __double2hiint(b)) & (int)0x80000000;
-    return __hiloint2double((__double2hiint(q) & 0x7fffffff) | s, __double2loint(q));
-}
-// i2: about 1 / (2 sqrt(x)), to a few ulps
-BH_HD inline double sqrt_rn(double x, double& i2) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    double g = x * y, h = 0.5 * y, r = fma(-g, h, 0.5);
-    g = fma(g, r, g); h = fma(h, r, h);
-    r = fma(-g, h, 0.5);
-    g = fma(g, r, g); h = fma(h, r, h);
-    i2 = h;
-    return fma(fma(-g, g, x), h, g);
-}
-#else
-BH_HD inline bool all_ones(double) { return false; }
-BH_HD inline double rcp_polish(double b, double) { return 1.0 / b; }
-BH_HD inline double rcp_rn(double b) { return 1.0 / b; }
-BH_HD inline double div_by(double a, double b, double) { return a / b; }
-BH_HD inline double sqrt_rn(double x, double& i2) { i2 = 0.5 / sqrt(x); return sqrt(x); }
-#endif
-
 BH_HD inline double f_df(double gamma, double xi, double Ssq, double Bsq, double SB,
                                        double Dn, double taun, double& df) {
     double Yi = SB * SB;
