@@ -961,17 +961,41 @@ __global__ void __launch_bounds__(FX_TPB) k_fx_pack(Grid G, const int32_t* items
     double* pf = pb + 3 * Q + face_off[b];
     WT* W = (WT*)G.W;
     const int si = bstride_i(B), sj = bstride_j(B);
+    // Bound: HBM.  Both sides are loaded in full before the first store: a load
+    // behind a store that may alias it waits for it, thirteen round trips per
+    // cell (176.6 MB each way at 128^3: pack 81 -> 61 us, unpack
+    // 87 -> 73; at 256^3, 1.41 GB, unpack 603 -> 486 us, 5.8 TB/s).
+    double u[5], f[3];
+    WT w[5];
     if (dir == 0) {
-        for (int v = 0; v < 5; v++) pu[v * Q + q] = G.U[v * N + c];
-        for (int v = 0; v < 5; v++) pw[v * Q + q] = W[v * N + c];
-        for (int d = 0; d < 3; d++) pb[d * Q + q] = G.Bf[d * N + c];
+#pragma unroll
+        for (int v = 0; v < 5; v++) u[v] = G.U[v * N + c];
+#pragma unroll
+        for (int v = 0; v < 5; v++) w[v] = W[v * N + c];
+#pragma unroll
+        for (int d = 0; d < 3; d++) f[d] = G.Bf[d * N + c];
+#pragma unroll
+        for (int v = 0; v < 5; v++) pu[v * Q + q] = u[v];
+#pragma unroll
+        for (int v = 0; v < 5; v++) pw[v * Q + q] = w[v];
+#pragma unroll
+        for (int d = 0; d < 3; d++) pb[d * Q + q] = f[d];
         if (i == n - 1) pf[j * n + k] = G.Bf[c + si];
         if (j == n - 1) pf[n * n + i * n + k] = G.Bf[N + c + sj];
         if (k == n - 1) pf[2 * n * n + i * n + j] = G.Bf[2 * N + c + 1];
     } else {
-        for (int v = 0; v < 5; v++) G.U[v * N + c] = pu[v * Q + q];
-        for (int v = 0; v < 5; v++) W[v * N + c] = pw[v * Q + q];
-        for (int d = 0; d < 3; d++) G.Bf[d * N + c] = pb[d * Q + q];
+#pragma unroll
+        for (int v = 0; v < 5; v++) u[v] = pu[v * Q + q];
+#pragma unroll
+        for (int v = 0; v < 5; v++) w[v] = pw[v * Q + q];
+#pragma unroll
+        for (int d = 0; d < 3; d++) f[d] = pb[d * Q + q];
+#pragma unroll
+        for (int v = 0; v < 5; v++) G.U[v * N + c] = u[v];
+#pragma unroll
+        for (int v = 0; v < 5; v++) W[v * N + c] = w[v];
+#pragma unroll
+        for (int d = 0; d < 3; d++) G.Bf[d * N + c] = f[d];
         if (i == n - 1) G.Bf[c + si] = pf[j * n + k];
         if (j == n - 1) G.Bf[N + c + sj] = pf[n * n + i * n + k];
         if (k == n - 1) G.Bf[2 * N + c + 1] = pf[2 * n * n + i * n + j];
