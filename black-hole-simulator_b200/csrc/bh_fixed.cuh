@@ -132,7 +132,23 @@ __device__ __forceinline__ void for_items(const Queue& q, Body body) {
     }
 }
 
+// ======================================================================
+// The step's kernels may be launched as programmatic dependents (fx_launch): a
+// kernel's CTAs may take their places once every CTA of the one before has
+// started, and wait here, before anything else, until it has finished and its
+// writes are visible.  That hides each launch and the filling of the SMs
+// behind the last wave of the kernel before.  Every thread of every kernel
+// begins with it: a kernel that ended without waiting would let the next one
+// pass the one before it.
+// ======================================================================
+__device__ __forceinline__ void after_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __global__ void k_fx_dt_init(double* dt) {
+    after_previous();
+    if (threadIdx.x) return;
     dt[0] = __longlong_as_double(0x7FF0000000000000LL);   // +inf
 }
 
@@ -265,6 +281,7 @@ __device__ inline void c2p_inputs(const Grid& G, const bh_fx_block& B, int i, in
 template <typename RT, typename WT, int MINB>
 __global__ void __launch_bounds__(FX_TPB, MINB) k_fx_c2p(FxPar P, Grid G, const int32_t* items, int stage,
                                                        int with_dt, Queue Q) {
+    after_previous();
     for_items(Q, [&](int t) FX_INLINE {
         const int32_t b = items[2 * t];
         const bh_fx_block B = G.blk[b];
@@ -381,6 +398,7 @@ __device__ inline int64_t bidx(const GhostSrc& b, int i, int j, int k) {
 }
 template <typename WT>
 __global__ void __launch_bounds__(FX_TPB, 8) k_fx_ghost(Grid G, const int32_t* items, int stage, int pass) {
+    after_previous();
     const int t = blockIdx.x;
     const int32_t b = items[2 * t];
     const bh_fx_block B = G.blk[b];
@@ -572,6 +590,7 @@ __device__ inline void face_flux(const FxPar& P, const Grid& G, const bh_fx_bloc
 
 template <typename RT, typename WT, typename FT, int MINB>
 __global__ void __launch_bounds__(FX_TPB, MINB) k_fx_flux(FxPar P, Grid G, const int32_t* items, int stage, Queue Q) {
+    after_previous();
     for_items(Q, [&](int t) FX_INLINE {
         const int32_t b = items[2 * t];
         const bh_fx_block B = G.blk[b];
@@ -629,6 +648,7 @@ __device__ inline int box_at(int a, int b, int c) { return ((a + 2) * FX_HJ + (b
 template <typename RT, typename WT, typename FT, int MINB>
 __global__ void __launch_bounds__(FX_TPB, MINB) k_fx_flux_tile(FxPar P, Grid G, const int32_t* items, int stage,
                                                              Queue Q) {
+    after_previous();
     __shared__ WT sW[8][FX_HBOX];
     for_items(Q, [&](int t) FX_INLINE {
         const int32_t b = items[2 * t];
@@ -743,6 +763,7 @@ __device__ inline void face_update(const Grid& G, int d, int64_t c, int si, int 
 // i in [0,n), j, k in [0,n], and alike), from the face fluxes
 template <typename FT>
 __global__ void __launch_bounds__(FX_TPB) k_fx_emf(Grid G, const int32_t* items, Queue Q) {
+    after_previous();
     for_items(Q, [&](int t) FX_INLINE {
         const int32_t b = items[2 * t];
         const bh_fx_block B = G.blk[b];
@@ -765,6 +786,7 @@ __global__ void __launch_bounds__(FX_TPB) k_fx_emf(Grid G, const int32_t* items,
 // field of the coarse side stays the mean of the fine faces (div B at
 // roundoff).  Levels differ by one at most, so one pass suffices.
 __global__ void __launch_bounds__(FX_TPB) k_fx_emf_fix(Grid G, const int32_t* items) {
+    after_previous();
     const int t = blockIdx.x;
     const int32_t b = items[2 * t];
     const bh_fx_block B = G.blk[b];
@@ -811,6 +833,7 @@ __global__ void __launch_bounds__(FX_TPB) k_fx_emf_fix(Grid G, const int32_t* it
 template <typename RT, typename WT, typename FT, int MINB, int PART>
 __global__ void __launch_bounds__(FX_TPB, MINB) k_fx_update(FxPar P, Grid G, const int32_t* items, int stage,
                                                       double cfl, Queue Q) {
+    after_previous();
     for_items(Q, [&](int t) FX_INLINE {
         const int32_t b = items[2 * t];
         const bh_fx_block B = G.blk[b];
@@ -947,6 +970,7 @@ __global__ void __launch_bounds__(FX_TPB, MINB) k_fx_update(FxPar P, Grid G, con
 template <typename WT>
 __global__ void __launch_bounds__(FX_TPB) k_fx_pack(Grid G, const int32_t* items, int nitem, const int64_t* face_off,
                                                     char* packed, int dir) {
+    after_previous();
     const int t = blockIdx.x;
     const int32_t b = items[2 * t];
     const bh_fx_block B = G.blk[b];
@@ -1251,6 +1275,27 @@ inline fx::Queue fx_q(const bh_fx_grid* g, int slot, int nitem) {
     if (!g->queue) return fx::Queue{nullptr, nullptr, nitem};
     return fx::Queue{g->queue + 2 * slot, g->queue + 2 * slot + 1, nitem};
 }
+// `ctas` CTAs of FX_TPB threads, as a programmatic dependent of the launch
+// before it in the stream (after_previous) where that pays: not into a graph,
+// whose nodes follow one another as closely without (step of 16^3 / 128^3
+// mixed, us: stream 124 / 1202 plain, 112 / 1190 dependent; graph 109 / 1181
+// plain, 113 / 1193 dependent), nor beyond 32768 CTAs, where the last wave is a
+// small part (192^3 3665 plain, 3672 dependent).
+template <typename... K, typename... A>
+inline void fx_launch(void (*kernel)(K...), int ctas, cudaStream_t st, const A&... args) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool known = !st || cudaStreamIsCapturing(st, &cap) == cudaSuccess;   // (the legacy stream never captures)
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3((unsigned)ctas);
+    c.blockDim = dim3(fx::FX_TPB);
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = known && cap == cudaStreamCaptureStatusNone && ctas <= 32768 ? 1 : 0;
+    cudaLaunchKernelEx(&c, kernel, (K)(args)...);
+}
 inline int fx_sms() {
     static int sms = 0;
     if (!sms) {
@@ -1354,9 +1399,9 @@ int fx_tune_get(int32_t kernel, int32_t* ctas) {
 int fx_prims(const bh_fx_params* P, const bh_fx_grid* g, int32_t stage, int32_t with_dt, void* s) {
     fx::FxPar p = fx::par_of(P);
     fx::Grid G = fx::grid_of(g);
-    if (with_dt) fx::k_fx_dt_init<<<1, 1, 0, fxs(s)>>>(g->dt);
+    if (with_dt) fx_launch(fx::k_fx_dt_init, 1, fxs(s), g->dt);
     if (g->nitem_cell) {
-#define L_(M) fx::k_fx_c2p<FRT, FRT, M><<<fx_grid((const void*)fx::k_fx_c2p<FRT, FRT, M>, g->nitem_cell, g), fx::FX_TPB, 0, fxs(s)>>>(p, G, g->items_cell, stage, with_dt, fx_q(g, QS_C2P, g->nitem_cell))
+#define L_(M) fx_launch(fx::k_fx_c2p<FRT, FRT, M>, fx_grid((const void*)fx::k_fx_c2p<FRT, FRT, M>, g->nitem_cell, g), fxs(s), p, G, g->items_cell, stage, with_dt, fx_q(g, QS_C2P, g->nitem_cell))
         FX_TUNED(fx_choose(BH_FX_TUNE_C2P, P, g), L_)
 #undef L_
     }
@@ -1369,7 +1414,7 @@ int fx_ghost_pass(const bh_fx_params*, const bh_fx_grid* g, int32_t stage, int32
     // between items makes its warps wait for the longest (three levels, FP64,
     // passes 0-2: 126 + 44 + 28 us persistent, 107 + 37 + 21 like this)
     if (g->nitem_ghost)
-        fx::k_fx_ghost<FRT><<<g->nitem_ghost, fx::FX_TPB, 0, fxs(s)>>>(G, g->items_ghost, stage, pass);
+        fx_launch(fx::k_fx_ghost<FRT>, g->nitem_ghost, fxs(s), G, g->items_ghost, stage, pass);
     return fx_launched();
 }
 int fx_ghosts(const bh_fx_params* P, const bh_fx_grid* g, int32_t stage, void* s) {
@@ -1382,11 +1427,11 @@ int fx_fluxes(const bh_fx_params* P, const bh_fx_grid* g, int32_t stage, void* s
     fx::FxPar p = fx::par_of(P);
     fx::Grid G = fx::grid_of(g);
     if (fx_choose(BH_FX_TUNE_STAGE, P, g)) {
-#define L_(M) fx::k_fx_flux_tile<FRT, FRT, FRT, M><<<fx_grid((const void*)fx::k_fx_flux_tile<FRT, FRT, FRT, M>, g->nitem_flux, g), fx::FX_TPB, 0, fxs(s)>>>(p, G, g->items_flux, stage, fx_q(g, QS_FLUX, g->nitem_flux))
+#define L_(M) fx_launch(fx::k_fx_flux_tile<FRT, FRT, FRT, M>, fx_grid((const void*)fx::k_fx_flux_tile<FRT, FRT, FRT, M>, g->nitem_flux, g), fxs(s), p, G, g->items_flux, stage, fx_q(g, QS_FLUX, g->nitem_flux))
         FX_TUNED(fx_choose(BH_FX_TUNE_FLUX, P, g), L_)
 #undef L_
     } else if (g->nitem_pos) {
-#define L_(M) fx::k_fx_flux<FRT, FRT, FRT, M><<<fx_grid((const void*)fx::k_fx_flux<FRT, FRT, FRT, M>, g->nitem_pos, g), fx::FX_TPB, 0, fxs(s)>>>(p, G, g->items_pos, stage, fx_q(g, QS_FLUX, g->nitem_pos))
+#define L_(M) fx_launch(fx::k_fx_flux<FRT, FRT, FRT, M>, fx_grid((const void*)fx::k_fx_flux<FRT, FRT, FRT, M>, g->nitem_pos, g), fxs(s), p, G, g->items_pos, stage, fx_q(g, QS_FLUX, g->nitem_pos))
         FX_TUNED(fx_choose(BH_FX_TUNE_FLUX, P, g), L_)
 #undef L_
     }
@@ -1398,19 +1443,19 @@ int fx_update_parts(const bh_fx_params* P, const bh_fx_grid* g, int32_t stage, i
     fx::FxPar p = fx::par_of(P);
     fx::Grid G = fx::grid_of(g);
     if (g->E && g->nitem_pos && (parts & 1))
-        fx::k_fx_emf<FRT><<<fx_grid((const void*)fx::k_fx_emf<FRT>, g->nitem_pos, g), fx::FX_TPB, 0, fxs(s)>>>(
-            G, g->items_pos, fx_q(g, QS_EMF, g->nitem_pos));
+        fx_launch(fx::k_fx_emf<FRT>, fx_grid((const void*)fx::k_fx_emf<FRT>, g->nitem_pos, g), fxs(s), G, g->items_pos,
+                  fx_q(g, QS_EMF, g->nitem_pos));
     if (!(parts & 2)) return fx_launched();
     if (g->E && g->nitem_pos && g->maxlevel > 0)   // (one CTA per item, as the ghost fill: most items have no work)
-        fx::k_fx_emf_fix<<<g->nitem_pos, fx::FX_TPB, 0, fxs(s)>>>(G, g->items_pos);
+        fx_launch(fx::k_fx_emf_fix, g->nitem_pos, fxs(s), G, g->items_pos);
     if (g->nitem_cell && fx_choose(BH_FX_TUNE_SPLIT, P, g)) {
-#define L_(M) fx::k_fx_update<FRT, FRT, FRT, M, 1><<<fx_grid((const void*)fx::k_fx_update<FRT, FRT, FRT, M, 1>, g->nitem_cell, g), fx::FX_TPB, 0, fxs(s)>>>(p, G, g->items_cell, stage, P->cfl, fx_q(g, QS_UPDATE, g->nitem_cell))
+#define L_(M) fx_launch(fx::k_fx_update<FRT, FRT, FRT, M, 1>, fx_grid((const void*)fx::k_fx_update<FRT, FRT, FRT, M, 1>, g->nitem_cell, g), fxs(s), p, G, g->items_cell, stage, P->cfl, fx_q(g, QS_UPDATE, g->nitem_cell))
         FX_TUNED(fx_choose(BH_FX_TUNE_UPDATE, P, g), L_)
 #undef L_
-        fx::k_fx_update<FRT, FRT, FRT, 8, 2><<<fx_grid((const void*)fx::k_fx_update<FRT, FRT, FRT, 8, 2>, g->nitem_cell, g), fx::FX_TPB, 0, fxs(s)>>>(
-            p, G, g->items_cell, stage, P->cfl, fx_q(g, QS_UPDATE_B, g->nitem_cell));
+        fx_launch(fx::k_fx_update<FRT, FRT, FRT, 8, 2>,
+                  fx_grid((const void*)fx::k_fx_update<FRT, FRT, FRT, 8, 2>, g->nitem_cell, g), fxs(s), p, G, g->items_cell, stage, P->cfl, fx_q(g, QS_UPDATE_B, g->nitem_cell));
     } else if (g->nitem_cell) {
-#define L_(M) fx::k_fx_update<FRT, FRT, FRT, M, 3><<<fx_grid((const void*)fx::k_fx_update<FRT, FRT, FRT, M, 3>, g->nitem_cell, g), fx::FX_TPB, 0, fxs(s)>>>(p, G, g->items_cell, stage, P->cfl, fx_q(g, QS_UPDATE, g->nitem_cell))
+#define L_(M) fx_launch(fx::k_fx_update<FRT, FRT, FRT, M, 3>, fx_grid((const void*)fx::k_fx_update<FRT, FRT, FRT, M, 3>, g->nitem_cell, g), fxs(s), p, G, g->items_cell, stage, P->cfl, fx_q(g, QS_UPDATE, g->nitem_cell))
         FX_TUNED(fx_choose(BH_FX_TUNE_UPDATE, P, g), L_)
 #undef L_
     }
@@ -1432,7 +1477,7 @@ int fx_step(const bh_fx_params* P, const bh_fx_grid* g, void* s) {
 int fx_pack_state(const bh_fx_grid* g, const int64_t* face_off, void* packed, int32_t dir, void* s) {
     fx::Grid G = fx::grid_of(g);
     if (g->nitem_cell)
-        fx::k_fx_pack<FRT><<<g->nitem_cell, fx::FX_TPB, 0, fxs(s)>>>(G, g->items_cell, g->nitem_cell, face_off,
+        fx_launch(fx::k_fx_pack<FRT>, g->nitem_cell, fxs(s), G, g->items_cell, g->nitem_cell, face_off,
                                                                      (char*)packed, dir);
     return fx_launched();
 }
