@@ -91,7 +91,6 @@ BH_FI float sqrt_(float x) { return sqrtf(x); }
 // ----------------------------------------------------------------------
 template <typename T, bool FAST>
 struct Ops {
-    static BH_FI void need(bool&, bool) {}
     static BH_FI T recip(T b) { return T(1) / b; }
     static BH_FI T quot(T a, T b) { return a / b; }
     static BH_FI T quot_by(T a, T b, T) { return a / b; }
@@ -153,7 +152,8 @@ BH_FI void ks_metric_ops(const FxPar& P, T x, T y, T z, KSb<T>& m, bool& ok) {
     using O = Ops<T, FAST>;
     const T a = T(P.a), a2 = a * a;
     T r2 = ks_r2(a, x, y, z);
-    O::need(ok, P.sane && r2 >= T(1e-60) && r2 <= T(1e60) && (z == T(0) || fabs_(z) >= T(1e-60)));
+    if constexpr (FAST)
+        O::need(ok, P.sane && r2 >= T(1e-60) && r2 <= T(1e60) && (z == T(0) || fabs_(z) >= T(1e-60)));
     T ir, r = O::root(r2, ir);
     T q = r2 * r2 + a2 * z * z;
     // on the disc z = 0, x^2 + y^2 <= a^2 (r = 0) the metric is flat
@@ -249,7 +249,7 @@ BH_FI void derive_ops(const KSm<RT>& m, RT gg, const RT* w, Derived<RT>& d, bool
     lower(m.g, ut, utl);
     RT u2 = utl[0] * ut[0] + utl[1] * ut[1] + utl[2] * ut[2];
     d.u2 = u2;
-    O::need(ok, u2 >= RT(0) && u2 <= RT(1e12));
+    if constexpr (FAST) O::need(ok, u2 >= RT(0) && u2 <= RT(1e12));
     RT iW;
     d.W = O::root(RT(1) + u2, iW);
     d.iW = iW;
@@ -321,7 +321,8 @@ BH_FI void signal_speeds_ops(const KSm<RT>& m, RT gamma, int dd, const RT* w, co
     using O = Ops<RT, FAST>;
     RT rhoh = d.rhoh;
     // c_s^2 + v_A^2 - c_s^2 v_A^2 with c_s^2 = Gamma p / (rho h), v_A^2 = b^2 / (rho h + b^2)
-    O::need(ok, d.b2 >= RT(0) && w[P_PRS] >= RT(1e-100) && rhoh + d.b2 <= RT(1e100) && rhoh >= RT(1e-100));
+    if constexpr (FAST)
+        O::need(ok, d.b2 >= RT(0) && w[P_PRS] >= RT(1e-100) && rhoh + d.b2 <= RT(1e100) && rhoh >= RT(1e-100));
     RT c2 = O::quot(gamma * w[P_PRS] + d.b2, rhoh + d.b2);
     c2 = fmin_(fmax_(c2, RT(0)), RT(1));
     RT v2 = RT(1) - d.iW * d.iW;
@@ -450,7 +451,7 @@ BH_FI RT hll_face_ops(const KSm<RT>& m, RT gamma, RT gg, int dd, const RT* wL, c
     RT sr = fmax_(fmax_(lpL, lpR), RT(0));
     RT ds = sr - sl;
     if (ds > RT(0)) {
-        O::need(ok, ds >= RT(1e-100) && ds <= RT(1e100));
+        if constexpr (FAST) O::need(ok, ds >= RT(1e-100) && ds <= RT(1e100));
         RT ids = O::recip(ds), ss = sr * sl;
         for (int v = 0; v < 8; v++) F[v] = (sr * FL[v] - sl * FR[v] + ss * (uR[v] - uL[v])) * ids;
     } else {
