@@ -22,7 +22,7 @@ import numpy as np
 import torch
 
 from bhgrid.blocks import (BLOCK_DTYPE, CHUNK, TILE_MIN, box_size, flux_items, ghost_depth,  # noqa: F401
-                           interior as _interior, leveled_blocks, uniform_blocks, work_items)
+                           interior as _interior, item_counts, leveled_blocks, uniform_blocks, work_items)
 
 from ._lib import BH_FP64, BH_FP64_FMA, BH_MIXED, BH_MC, BH_MINMOD, BH_PPM, BH_VANLEER, BhError, check, lib
 
@@ -44,7 +44,8 @@ class BhFxGrid(C.Structure):
                 ("items_pos", _vp), ("nitem_pos", _i32), ("items_ghost", _vp), ("nitem_ghost", _i32),
                 ("ncell", _i64), ("U", _vp), ("U1", _vp), ("W", _vp), ("Bf", _vp), ("Bf1", _vp), ("F", _vp),
                 ("dt", _vp), ("count", _vp), ("err", _vp), ("E", _vp), ("maxlevel", _i32), ("queue_ctas", _i32), ("queue", _vp),
-                ("items_flux", _vp), ("nitem_flux", _i32), ("ghost_depth", _i32)]
+                ("items_flux", _vp), ("nitem_flux", _i32), ("ghost_depth", _i32),
+                ("rule_cell", _i32), ("rule_pos", _i32), ("rule_flux", _i32)]
 
 
 class BhFxTorus(C.Structure):
@@ -163,6 +164,8 @@ class FxGrid:
             emf_arrays = self.maxlevel > 0
         self.E = torch.zeros((3, N), dtype=torch.float64, device=dev) if emf_arrays else None
         self.queue = torch.zeros(2 * QSLOTS, dtype=torch.int32, device=dev) if persistent else None
+        self._rule = (0, 0, 0)
+        self._tile_min = tile_min
         self._refresh()
 
     @classmethod
@@ -186,8 +189,24 @@ class FxGrid:
                            _ptr(it["ghost"]), it["ghost"].shape[0], self.ncell,
                            _ptr(self.U), _ptr(self.U1), _ptr(self.W), _ptr(self.Bf), _ptr(self.Bf1), _ptr(self.F),
                            _ptr(self.dt), _ptr(self.count), _ptr(self.err), _ptr(self.E), self.maxlevel, 0, _ptr(self.queue),
-                           _ptr(it["flux"]), it["flux"].shape[0], self.ghost_depth)
+                           _ptr(it["flux"]), it["flux"].shape[0], self.ghost_depth, *self._rule)
         self._p = self.params.cstruct()
+
+    def launch_as_share_of(self, blocks: np.ndarray, parts: int):
+        """The launch rules go by the mean share of the domain ``blocks`` cut
+        into ``parts`` (not by this grid's own work items): the same kernels
+        on every rank (ShardedFxGrid calls it)."""
+        c = item_counts(blocks, self._tile_min)
+        self._rule = tuple(-(-c[k] // parts) for k in ("cell", "pos", "flux"))
+        self._refresh()
+
+    def launch_choice(self, kernel: str) -> int:
+        """What a launch on this grid takes for a knob of TUNE_KNOBS (by the
+        process's setting or by rule)."""
+        v = _i32()
+        check(lib.bh_fx_tune_choice(C.byref(self._p), C.byref(self._g), TUNE_KNOBS.index(kernel), C.byref(v)),
+              "bh_fx_tune_choice")
+        return int(v.value)
 
     @property
     def precision(self):
@@ -425,6 +444,8 @@ TUNE_KNOBS = TUNE_KERNELS + ("stage", "split")   # 1 = the staged flux kernel; t
 TUNE_CANDIDATES = (1, 3, 4, 5, 6, 7, 8)
 lib.bh_fx_tune_set.argtypes = [_i32, _i32, _i32]
 lib.bh_fx_tune_get.argtypes = [_i32, _i32, C.POINTER(_i32)]
+lib.bh_fx_tune_choice.argtypes = [C.POINTER(BhFxParams), C.POINTER(BhFxGrid), _i32, C.POINTER(_i32)]
+lib.bh_fx_tune_choice.restype = C.c_int
 lib.bh_fx_tune_set.restype = C.c_int
 lib.bh_fx_tune_get.restype = C.c_int
 

@@ -47,6 +47,10 @@ class ShardedFxGrid:
         self.maxlevel = int(blocks["level"].max())
         self.local = local_grid(blocks, nbr, self.owner, self.rank)
         self.grid = grid_factory(self.local.blocks, self.local.nbr, self.local.nown, self.maxlevel)
+        if hasattr(self.grid, "launch_as_share_of"):
+            # the ranks' work lists differ in length: one choice of kernels for
+            # all of them, or a face shared by two ranks rounds in two ways
+            self.grid.launch_as_share_of(blocks, self.world)
         self.global_blocks = blocks
         plan = exchange_plan(blocks, nbr, self.owner, self.rank)
         dev = self._t("W").device

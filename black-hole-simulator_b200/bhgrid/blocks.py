@@ -99,6 +99,16 @@ def flux_items(blocks: np.ndarray, tile_min: int = TILE_MIN) -> np.ndarray:
     return np.concatenate(out).astype(np.int32)
 
 
+def item_counts(blocks: np.ndarray, tile_min: int = TILE_MIN) -> dict:
+    """Lengths of the work lists of ``blocks`` ('cell', 'pos', 'flux')."""
+    n, k = np.unique(np.asarray(blocks["n"]), return_counts=True)
+    n, k = n.astype(np.int64), k.astype(np.int64)
+    pos = -(-(n + 2) ** 3 // CHUNK)
+    tiles = np.prod([-(-(n + 2) // t) for t in TILE], 0)
+    return {"cell": int((-(-n ** 3 // CHUNK) * k).sum()), "pos": int((pos * k).sum()),
+            "flux": int((np.where(n >= tile_min, tiles, pos) * k).sum())}
+
+
 def flux_item_positions(n: int, e: int) -> np.ndarray:
     """Positions (i, j, k) in [-1, n]^3 that item e of a block of n cells
     covers (the kernel's decode; positions beyond n are masked)."""

@@ -251,6 +251,10 @@ int bh_fx_tune_get(int32_t precision, int32_t kernel, int32_t* ctas) {
     default: return BH_EINVAL;
     }
 }
+int bh_fx_tune_choice(const bh_fx_params* P, const bh_fx_grid* g, int32_t kernel, int32_t* choice) {
+    if (!P || !g || !choice || P->precision < BH_FP64 || P->precision > BH_MIXED) return BH_EINVAL;
+    FX_DISPATCH(P, fx_tune_choice(P, g, kernel, choice));
+}
 int bh_fx_pack_state(const bh_fx_params* P, const bh_fx_grid* g, const int64_t* face_off, void* packed, int32_t dir,
                      void* stream) {
     if (fx_bad(P, g) || !face_off || !packed || (dir != 0 && dir != 1)) return BH_EINVAL;

@@ -1371,22 +1371,28 @@ namespace {
 //             second launch costs more: 16^3 12 -> 17).
 // A grid of up to four items per SM takes no cap: nothing waits for a slot,
 // and a capped kernel's spills only lengthen it (16^3 step 134 -> 144).
+// A grid that is one rank's share of a domain brings the counts to go by (the
+// same on every rank): its own differ from the other ranks', and kernels chosen
+// by them would round a face shared by two ranks in two ways.
 int fx_choose(int kernel, const bh_fx_params* P, const bh_fx_grid* g) {
     const int set = fx_tune_tab[kernel];
     constexpr bool F32 = sizeof(FRT) < sizeof(double);
+    const bool own = !g->rule_cell && !g->rule_pos && !g->rule_flux;
+    const int cell = own ? g->nitem_cell : g->rule_cell, pos = own ? g->nitem_pos : g->rule_pos,
+              flux = own ? g->nitem_flux : g->rule_flux;
     const bool staged = fx_tune_tab[BH_FX_TUNE_STAGE] == FX_AUTO_FORM
-                            ? g->nitem_flux > g->nitem_pos && 10 * (int64_t)g->nitem_flux <= 11 * (int64_t)g->nitem_pos
+                            ? flux > pos && 10 * (int64_t)flux <= 11 * (int64_t)pos
                             : fx_tune_tab[BH_FX_TUNE_STAGE] == 1;
     const int few = 4 * fx_sms();   // work items
     switch (kernel) {
     case BH_FX_TUNE_STAGE: return staged && g->nitem_flux && P->limiter != fx::FX_PPM;
     case BH_FX_TUNE_SPLIT:
-        return set != FX_AUTO_FORM ? set : (g->E || g->nitem_cell >= (F32 ? 8192 : 2048));
-    case BH_FX_TUNE_C2P: return set != FX_AUTO ? set : (g->nitem_cell <= few ? 1 : (F32 ? 7 : 6));
+        return set != FX_AUTO_FORM ? set : (g->E || cell >= (F32 ? 8192 : 2048));
+    case BH_FX_TUNE_C2P: return set != FX_AUTO ? set : (cell <= few ? 1 : (F32 ? 7 : 6));
     case BH_FX_TUNE_FLUX:
         if (set != FX_AUTO) return set;
-        return g->nitem_pos <= few ? 1 : (F32 ? 8 : (staged && P->limiter != fx::FX_PPM ? 4 : 5));
-    default: return set != FX_AUTO ? set : (g->nitem_cell <= few ? 1 : (F32 ? 8 : 4));
+        return pos <= few ? 1 : (F32 ? 8 : (staged && P->limiter != fx::FX_PPM ? 4 : 5));
+    default: return set != FX_AUTO ? set : (cell <= few ? 1 : (F32 ? 8 : 4));
     }
 }
 }  // namespace
@@ -1403,6 +1409,11 @@ int fx_tune_set(int32_t kernel, int32_t ctas) {
 int fx_tune_get(int32_t kernel, int32_t* ctas) {
     if (kernel < 0 || kernel >= BH_FX_TUNE_N || !ctas) return BH_EINVAL;
     *ctas = fx_tune_tab[kernel];
+    return BH_OK;
+}
+int fx_tune_choice(const bh_fx_params* P, const bh_fx_grid* g, int32_t kernel, int32_t* choice) {
+    if (kernel < 0 || kernel >= BH_FX_TUNE_N) return BH_EINVAL;
+    *choice = fx_choose(kernel, P, g);
     return BH_OK;
 }
 

@@ -463,6 +463,13 @@ typedef struct bh_fx_grid {
     int32_t ghost_depth;         /* ghost layers the fill covers (and items_ghost
                                     lists): 2 (0 reads as 2), or 3, which BH_PPM
                                     requires                                        */
+    int32_t rule_cell, rule_pos, rule_flux;  /* the numbers of work items that the
+                                    launch rules (BH_FX_TUNE_*) go by; all 0:
+                                    nitem_cell, nitem_pos, nitem_flux.  The grids of
+                                    one domain's ranks set the same numbers, so that
+                                    every rank runs the same kernels (in the
+                                    contracted variants other kernels round
+                                    otherwise)                                      */
 } bh_fx_grid;
 #define BH_FX_QSLOTS 7
 
@@ -482,6 +489,10 @@ enum { BH_FX_TUNE_C2P = 0, BH_FX_TUNE_FLUX = 1, BH_FX_TUNE_UPDATE = 2, BH_FX_TUN
        BH_FX_TUNE_N = 5 };
 int bh_fx_tune_set(int32_t precision, int32_t kernel, int32_t ctas_per_sm);
 int bh_fx_tune_get(int32_t precision, int32_t kernel, int32_t *ctas_per_sm);
+/* what a launch with P on g takes for `kernel`, by the knob or by rule: CTAs
+ * per SM (1, 3..8), or 0/1 for BH_FX_TUNE_STAGE and BH_FX_TUNE_SPLIT.  Reads
+ * P's precision and limiter and g's counts, limits and E only; no launch. */
+int bh_fx_tune_choice(const bh_fx_params *P, const bh_fx_grid *g, int32_t kernel, int32_t *choice);
 
 /* one RK2 step: con2prim (+ CFL reduction), ghost fill, fluxes, update, twice */
 int bh_fx_step(const bh_fx_params *P, const bh_fx_grid *g, void *stream);
