@@ -45,7 +45,7 @@ class BhFxGrid(C.Structure):
                 ("ncell", _i64), ("U", _vp), ("U1", _vp), ("W", _vp), ("Bf", _vp), ("Bf1", _vp), ("F", _vp),
                 ("dt", _vp), ("count", _vp), ("err", _vp), ("E", _vp), ("maxlevel", _i32), ("queue_ctas", _i32), ("queue", _vp),
                 ("items_flux", _vp), ("nitem_flux", _i32), ("ghost_depth", _i32),
-                ("rule_cell", _i32), ("rule_pos", _i32), ("rule_flux", _i32)]
+                ("rule_cell", _i32), ("rule_pos", _i32), ("rule_flux", _i32), ("rule_tile", _i32)]
 
 
 class BhFxTorus(C.Structure):
@@ -164,7 +164,7 @@ class FxGrid:
             emf_arrays = self.maxlevel > 0
         self.E = torch.zeros((3, N), dtype=torch.float64, device=dev) if emf_arrays else None
         self.queue = torch.zeros(2 * QSLOTS, dtype=torch.int32, device=dev) if persistent else None
-        self._rule = (0, 0, 0)
+        self._rule = (0, 0, 0, item_counts(act, tile_min)["tile"])
         self._tile_min = tile_min
         self._refresh()
 
@@ -197,7 +197,7 @@ class FxGrid:
         into ``parts`` (not by this grid's own work items): the same kernels
         on every rank (ShardedFxGrid calls it)."""
         c = item_counts(blocks, self._tile_min)
-        self._rule = tuple(-(-c[k] // parts) for k in ("cell", "pos", "flux"))
+        self._rule = tuple(-(-c[k] // parts) for k in ("cell", "pos", "flux", "tile"))
         self._refresh()
 
     def launch_choice(self, kernel: str) -> int:

@@ -100,13 +100,15 @@ def flux_items(blocks: np.ndarray, tile_min: int = TILE_MIN) -> np.ndarray:
 
 
 def item_counts(blocks: np.ndarray, tile_min: int = TILE_MIN) -> dict:
-    """Lengths of the work lists of ``blocks`` ('cell', 'pos', 'flux')."""
+    """Lengths of the work lists of ``blocks`` ('cell', 'pos', 'flux') and the
+    tiles among the last ('tile')."""
     n, k = np.unique(np.asarray(blocks["n"]), return_counts=True)
     n, k = n.astype(np.int64), k.astype(np.int64)
     pos = -(-(n + 2) ** 3 // CHUNK)
     tiles = np.prod([-(-(n + 2) // t) for t in TILE], 0)
     return {"cell": int((-(-n ** 3 // CHUNK) * k).sum()), "pos": int((pos * k).sum()),
-            "flux": int((np.where(n >= tile_min, tiles, pos) * k).sum())}
+            "flux": int((np.where(n >= tile_min, tiles, pos) * k).sum()),
+            "tile": int((np.where(n >= tile_min, tiles, 0) * k).sum())}
 
 
 def flux_item_positions(n: int, e: int) -> np.ndarray:

@@ -1358,9 +1358,20 @@ namespace {
 // former default), over the 128^3 torus, 96^3 in 32^3 blocks and 512 blocks of
 // 8^3 to 32^3 (lev):
 //   con2prim  7 (mixed), 6: 128^3 237 -> 122 / 337 -> 197, lev 175 -> 105 / 241 -> 149.
-//   fluxes    the stencil staged where the tiles pad the positions by at most
-//             a tenth (blocks of ~100^3 on): 128^3 (8 %) 275 against 292 /
-//             542 against 562 unstaged, 64^3 (16 %) 45 against 42 / 94 against 87.
+//   fluxes    the stencil staged in shared memory by what the step takes then,
+//             not the launch alone (128^3 269 against 285 / 534 against 560
+//             unstaged): the update that follows finds less of a small grid's
+//             fluxes in L2 when they were written tile by tile.  Step staged /
+//             unstaged, mixed, FP64 (FMA in brackets):
+//               tiles fit exactly (n + 2 a multiple of 8): 70^3 1.05, 1.08
+//               (1.08); 94^3 1.00, .99 (1.02); 102^3 .99, .97 (1.01); 110^3
+//               .99, .97 (1.00); 126^3 .98, .95 (.99); 8 of 86^3 .96, .94 (.96);
+//               tiles pad by 5 to 10 %: 68^3 1.05, 1.10 (1.09); 92^3 1.02, 1.02
+//               (1.04); 104^3 1.02, 1.01 (1.04); 112^3 1.01, 1.00 (1.03); 124^3
+//               .99, .98 (1.01); 128^3 1.00, .99 (1.02); 160^3 .98, .97 (1.00); 8
+//               of 92^3 .98, .97 (.99); by 16 %: 8 of 64^3 1.03, 1.03 (1.06).
+//             Hence exact fits from 8192 items on (FMA 12288), padded tiles up
+//             to a tenth from 14336 on (FMA not at all).
 //             Resident CTAs 8 in FP32 (128^3 365 -> 275, PPM 540 -> 431);
 //             in FP64 4 staged (697 -> 542) and 5 unstaged (782 -> 562, PPM
 //             1082 -> 801): more would spill.
@@ -1380,9 +1391,16 @@ int fx_choose(int kernel, const bh_fx_params* P, const bh_fx_grid* g) {
     const bool own = !g->rule_cell && !g->rule_pos && !g->rule_flux;
     const int cell = own ? g->nitem_cell : g->rule_cell, pos = own ? g->nitem_pos : g->rule_pos,
               flux = own ? g->nitem_flux : g->rule_flux;
-    const bool staged = fx_tune_tab[BH_FX_TUNE_STAGE] == FX_AUTO_FORM
-                            ? flux > pos && 10 * (int64_t)flux <= 11 * (int64_t)pos
-                            : fx_tune_tab[BH_FX_TUNE_STAGE] == 1;
+#if defined(BH_RCP)   // (the contracted variants)
+    constexpr bool FMA64 = !F32;
+#else
+    constexpr bool FMA64 = false;
+#endif
+    const bool tiles = g->rule_tile > 0 || flux > pos, fit = flux == pos;
+    const bool pays = fit ? pos >= (FMA64 ? 12288 : 8192)
+                          : !FMA64 && pos >= 14336 && 10 * (int64_t)flux <= 11 * (int64_t)pos;
+    const bool staged = fx_tune_tab[BH_FX_TUNE_STAGE] == FX_AUTO_FORM ? tiles && pays
+                                                                      : fx_tune_tab[BH_FX_TUNE_STAGE] == 1;
     const int few = 4 * fx_sms();   // work items
     switch (kernel) {
     case BH_FX_TUNE_STAGE: return staged && g->nitem_flux && P->limiter != fx::FX_PPM;

@@ -470,6 +470,9 @@ typedef struct bh_fx_grid {
                                     every rank runs the same kernels (in the
                                     contracted variants other kernels round
                                     otherwise)                                      */
+    int32_t rule_tile;           /* the tiles among the rules' items_flux (0: taken to
+                                    be there where they are more than items_pos, which
+                                    tiles that fit their blocks exactly are not)    */
 } bh_fx_grid;
 #define BH_FX_QSLOTS 7
 

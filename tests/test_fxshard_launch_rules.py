@@ -22,7 +22,8 @@ def test_item_counts_are_the_lists_lengths():
         for tile_min in (16, 64):
             c = item_counts(blocks, tile_min)
             assert c["cell"] == len(work_items(blocks, "cell")) and c["pos"] == len(work_items(blocks, "pos"))
-            assert c["flux"] == len(flux_items(blocks, tile_min))
+            flux = flux_items(blocks, tile_min)
+            assert c["flux"] == len(flux) and c["tile"] == (flux[:, 1] >= 0).sum()
 
 
 def _worker(rank, world, port, out_dir):
