@@ -1380,8 +1380,14 @@ namespace {
 //             248) and on grids of 8192 items, in FP64 2048, or more (128^3
 //             169 -> 166 a stage / 255 -> 223, 64^3 40 -> 38; below that the
 //             second launch costs more: 16^3 12 -> 17).
-// A grid of up to four items per SM takes no cap: nothing waits for a slot,
-// and a capped kernel's spills only lengthen it (16^3 step 134 -> 144).
+// A grid whose items are all resident at once without a cap takes none: nothing
+// waits for a slot, and a capped kernel's spills only lengthen it.  In FP64 the
+// uncapped kernels (172 to 246 registers) keep 2 CTAs per SM: step uncapped /
+// capped 16^3 90 / 99 us, 30^3 (211 cell items, 256 of positions) 126 / 141;
+// 32^3 (256, 308) 137 without, 124 with all caps, 116 with the fluxes' alone;
+// 36^3 (365, 429) 174 / 151, 40^3 190 / 162.  In FP32 the flux kernel keeps 4
+// and the line is there for all: 32^3 98 / 107, 36^3 142 / 146, 40^3 (500, 579)
+// 132 / 132, 44^3 (666, 761) 167 / 143.
 // A grid that is one rank's share of a domain brings the counts to go by (the
 // same on every rank): its own differ from the other ranks', and kernels chosen
 // by them would round a face shared by two ranks in two ways.
@@ -1401,7 +1407,7 @@ int fx_choose(int kernel, const bh_fx_params* P, const bh_fx_grid* g) {
                           : !FMA64 && pos >= 14336 && 10 * (int64_t)flux <= 11 * (int64_t)pos;
     const bool staged = fx_tune_tab[BH_FX_TUNE_STAGE] == FX_AUTO_FORM ? tiles && pays
                                                                       : fx_tune_tab[BH_FX_TUNE_STAGE] == 1;
-    const int few = 4 * fx_sms();   // work items
+    const int few = (F32 ? 4 : 2) * fx_sms();   // work items
     switch (kernel) {
     case BH_FX_TUNE_STAGE: return staged && g->nitem_flux && P->limiter != fx::FX_PPM;
     case BH_FX_TUNE_SPLIT:

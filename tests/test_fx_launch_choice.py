@@ -61,6 +61,19 @@ def test_grids_bring_their_tiles():
     assert g._g.nitem_flux == g._g.nitem_pos == g._g.rule_tile == 2916
 
 
+def test_caps_where_the_uncapped_kernels_would_queue():
+    """no cap up to the CTAs the uncapped kernels keep resident: 2 per SM in
+    FP64, 4 in FP32 (a host without a GPU counts as one SM)"""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count if torch.cuda.is_available() else 1
+    for prec, per_sm, caps in (("mixed", 4, (7, 8, 8)), ("fp64", 2, (6, 5, 4)), ("fp64-fma", 2, (6, 5, 4))):
+        for items, want in ((per_sm * sms, (1, 1, 1)), (per_sm * sms + 1, caps)):
+            c = dict(cell=items, pos=items, flux=items, tile=0)
+            assert tuple(choice(k, prec, c) for k in ("c2p", "flux", "update")) == want
+            c["cell"] = 1     # (each kernel by its own list)
+            assert (choice("c2p", prec, c), choice("flux", prec, c)) == (1, want[1])
+
+
 @pytest.mark.gpu
 def test_exact_tiles_take_the_staged_fluxes_with_the_same_bits():
     import torch
