@@ -450,7 +450,8 @@ BH_HD inline bool fdf_fast(double gamma, double xi, double Ssq, double Bsq, doub
 // it the signs agree, and near om = 0 or p = 0, where fres takes its
 // constant branches (v^2 >= 1 and p < 0 count as positive), the decision
 // needs the same margin.  Anything irregular (NaN, overflow, xi or D not
-// positive) goes to fres.
+// positive, gamma <= 1, where g and with it the margin change sign) goes to
+// fres.
 //   Bound: FP64 latency of the con2prim kernels.  The reciprocal variants
 // keep fres, which has one division and one square root there.
 BH_HD inline double rcp_near(double x) {   // 1/x within a few ulps, x normal
@@ -486,7 +487,7 @@ BH_HD inline double fsgn(double gamma, double xi, double Ssq, double Bsq, double
 #ifndef BH_RCP
     const double U64 = 64.0 * 1.1102230246251565e-16;
     const double Yi = SB * SB, K = Bsq, X = xi * xi, xK = xi + K, Dv = X + xK * xK, XD = X * Dv;
-    if (XD > 1e-280 && XD < 1e300 && xi > 0.0 && Dn > 0.0) {
+    if (XD > 1e-280 && XD < 1e300 && xi > 0.0 && Dn > 0.0 && gamma > 1.0) {
         const double r = rcp_near(XD), iDv = X * r, hX = 0.5 * Dv * r;   // 1 / Dv, 1 / (2 X)
         const double n1 = Ssq * X, n2 = Yi * (2.0 * xi + K);
         const double om = 1.0 - (n1 + n2) * iDv, A = 1.0 + (fabs(n1) + fabs(n2)) * iDv;
@@ -643,10 +644,10 @@ struct CtopState {
 //   f(x) = x - tau - D - [g (x om - D sqrt(om)) + K om / 2 + Yi / (2 x^2)]
 // is positive, and stays so for every larger x (the constant branches
 // v^2 >= 1 and p < 0 are positive too): there the bracket's growth needs no
-// evaluation.  The 1e-9 slack is far above the residual's rounding.
+// evaluation.  It takes 0 < g < 1, which is gamma > 1.  The 1e-9 slack is far above the residual's rounding.
 BH_HD inline bool positive_above(double gamma, double x, double Ssq, double Bsq, double SB, double D, double tau) {
     const double g = (gamma - 1.0) / gamma;
-    return D > 0.0 && D < 1e40 && Ssq >= 0.0 && Bsq >= 0.0 && x > 1e-30 && x < 1e48 &&
+    return gamma > 1.0 && D > 0.0 && D < 1e40 && Ssq >= 0.0 && Bsq >= 0.0 && x > 1e-30 && x < 1e48 &&
            x * (1.0 - g) * (1.0 - 1e-9) > (fabs(tau) + D + 0.5 * Bsq) * (1.0 + 1e-9) + SB * SB / (x * x);
 }
 // pre[5] (may be null) receives D, tau, Ssq, Bsq, SB of the preamble; xi0:
