@@ -93,6 +93,7 @@ template <typename T, bool FAST>
 struct Ops {
     static BH_FI T recip(T b) { return T(1) / b; }
     static BH_FI T quot(T a, T b) { return a / b; }
+    static BH_FI T quot_pos(T a, T b) { return a / b; }   // a, b > 0
     static BH_FI T quot_by(T a, T b, T) { return a / b; }
     static BH_FI T quot_near(T a, T b, T) { return a / b; }
     static BH_FI T root(T x, T& inv) { T s = sqrt_(x); inv = T(1) / s; return s; }
@@ -103,13 +104,14 @@ struct Ops<double, true> {
     static BH_FI void need(bool& ok, bool c) { ok = ok && c; }
     static BH_FI double recip(double b) { return bh::rcp_any(b); }
     static BH_FI double quot(double a, double b) { return bh::div_by(a, b, bh::rcp_any(b)); }
+    static BH_FI double quot_pos(double a, double b) { return bh::div_pos(a, b, bh::rcp_any(b)); }
     static BH_FI double quot_by(double a, double b, double y) { return bh::div_by(a, b, y); }   // y = 1 / b
     static BH_FI double quot_near(double a, double b, double y) {                               // y near 1 / b
-        return bh::div_by(a, b, bh::rcp_polish_any(b, y));
+        return bh::div_by(a, b, bh::rcp_refine_any(b, y));
     }
     static BH_FI double root(double x, double& inv) {
         double i2, s = bh::sqrt_rn(x, i2);
-        inv = bh::rcp_polish_any(s, 2.0 * i2);
+        inv = bh::rcp_refine_any(s, 2.0 * i2);
         return s;
     }
     static BH_FI double root0(double x, bool& ok) {   // x >= 0
@@ -323,7 +325,7 @@ BH_FI void signal_speeds_ops(const KSm<RT>& m, RT gamma, int dd, const RT* w, co
     // c_s^2 + v_A^2 - c_s^2 v_A^2 with c_s^2 = Gamma p / (rho h), v_A^2 = b^2 / (rho h + b^2)
     if constexpr (FAST)
         O::need(ok, d.b2 >= RT(0) && w[P_PRS] >= RT(1e-100) && rhoh + d.b2 <= RT(1e100) && rhoh >= RT(1e-100));
-    RT c2 = O::quot(gamma * w[P_PRS] + d.b2, rhoh + d.b2);
+    RT c2 = O::quot_pos(gamma * w[P_PRS] + d.b2, rhoh + d.b2);
     c2 = fmin_(fmax_(c2, RT(0)), RT(1));
     RT v2 = RT(1) - d.iW * d.iW;
     RT vd = d.v[dd];

@@ -403,17 +403,18 @@ BH_HD inline bool fdf_fast(double gamma, double xi, double Ssq, double Bsq, doub
     const double Yi = SB * SB, K = Bsq, X = xi * xi, xipK = xi + K;
     const double N = Ssq * X + Yi * (2.0 * xi + K), Dv = X + xipK * xipK;
     if (all_ones(Dv)) return false;
-    const double vsq = div_by(N, Dv, rcp_rn(Dv));
+    // (S^2, B^2, (S.B)^2, D and xi are no negative numbers here: div_pos)
+    const double vsq = div_pos(N, Dv, rcp_rn(Dv));
     if (vsq >= 1.0) { f = 1e30; df = 0.0; return true; }
     const double om = 1.0 - vsq, ltz2 = rcp_rn(om);   // om in [2^-53, 1]
     double i2l;
     const double ltz = sqrt_rn(ltz2, i2l);
-    const double il = rcp_polish(ltz, 2.0 * i2l), il2 = rcp_polish(ltz2, om);
-    const double rho = div_by(Dn, ltz, il);
+    const double il = rcp_refine(ltz, 2.0 * i2l), il2 = rcp_polish(ltz2, om);
+    const double rho = div_pos(Dn, ltz, il);
     const double G = gamma - 1.0, gg = G / gamma;
-    const double p = gg * (div_by(xi, ltz2, il2) - rho);
+    const double p = gg * (div_pos(xi, ltz2, il2) - rho);
     const double iX = rcp_rn(X);
-    const double pstar = p + div_by(K, 2 * ltz2, 0.5 * il2) + div_by(Yi, 2 * X, 0.5 * iX);
+    const double pstar = p + div_pos(K, 2 * ltz2, 0.5 * il2) + div_pos(Yi, 2 * X, 0.5 * iX);
     const double dN = 2.0 * Ssq * xi + 2.0 * Yi;
     const double dM = 2.0 * xi * xipK * xipK + 2.0 * X * X;
     const double Mq = X * xipK * xipK, M2 = Mq * Mq;
@@ -424,12 +425,12 @@ BH_HD inline bool fdf_fast(double gamma, double xi, double Ssq, double Bsq, doub
         return false;
     if (p < 0.0 || rho < 0.0) { f = 1e32; df = 0.0; return true; }
     f = xi - taun - Dn - pstar;
-    const double il4 = rcp_polish(l4, il2 * il2);
+    const double il4 = rcp_refine(l4, il2 * il2);
     const double dltz2 = ltz2 * ltz2 * dvv;
     const double dltz = div_by(dltz2, 2.0 * ltz, 0.5 * il);
     const double dp = gg * (il2 - div_by(xi * dltz2, l4, il4) + div_by(Dn * dltz, ltz2, il2));
-    const double ixX = rcp_polish(xX, xi * iX * iX);
-    const double dpstar = dp - div_by(K * dltz2, 2.0 * ltz2 * ltz2, 0.5 * il4) - div_by(Yi, xX, ixX);
+    const double ixX = rcp_refine(xX, xi * iX * iX);
+    const double dpstar = dp - div_by(K * dltz2, 2.0 * ltz2 * ltz2, 0.5 * il4) - div_pos(Yi, xX, ixX);
     df = 1 - dpstar;
     return true;
 }
