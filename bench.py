@@ -62,6 +62,17 @@ LO, HI = -40.0, 40.0
 TORUS = dict(r_in=6.0, r_max=12.0, kappa=1e-3, beta=100.0, noise=0.04, seed=1)
 STEP_BYTES = 296          # algorithmic HBM bytes per zone-update of an RK2 step
 LAUNCHES_PER_STEP = 9     # dt init, then con2prim, ghosts, fluxes, update per stage (+1 per stage: split update)
+
+
+def step_launches(grid):
+    """Kernel launches of one step of a one-level grid, by what it runs."""
+    return LAUNCHES_PER_STEP + (2 if grid.launch_choice("split") else 0)
+
+
+def flux_kernel(grid):
+    return "k_fx_flux_tile" if grid.launch_choice("stage") else "k_fx_flux"
+
+
 # DRAM bytes (read + write) per launch of the mixed variant's step kernels at
 # 128^3, from the ncu capture summarised in profiles/kernels_torus_128cube.md
 # (the update as its two kernels, cells + faces: the autotuner's choice there)
@@ -536,7 +547,7 @@ def con2prim_batch(n_cells=1 << 24, reps=3):
         fail_t = (st != 1) & (stt_ != 1)
         out["mlp_guess"]["tensor_core"] = {
             "kernels": "k_guess_tc (metric, preamble, network as tcgen05.mma BF16 -> FP32 in TMEM, 128-cell "
-                       "tiles, persistent CTAs) + k_ctop_guess (Newton / Brent, one thread per cell)",
+                       "tiles, persistent CTAs) + k_ctop (Newton / Brent, lanes taking up cells as others end)",
             "ms": mst, "guess_kernel_ms": mst - ms_newton, "newton_kernel_ms": ms_newton,
             "cells_per_s": n_cells / (mst / 1e3), "speedup_vs_plain": ms / mst,
             "mean_newton_iters_where_both_recover": {"plain": float(it[both_t].mean()),
@@ -678,6 +689,7 @@ def run_ours(args):
     ms_mixed, clocks = timed_steps(g, args.steps, warm, dist, clocks_uuid=uuid or "", restart=restart_torus(g))
     counters = g.counters()
     divb_after = g.divb()
+    launches, flux_k = step_launches(g) * args.steps, flux_kernel(g)
     pieces = {"mixed": piece_ms(g)}
     ms_e2e, ms_e2e_serial, nbytes = e2e_measure(args, g, dist)
     del g
@@ -725,8 +737,6 @@ def run_ours(args):
         top_ms = pieces["mixed"][top]
         byts = alg_bytes(top, args.block, 4) * nblk
         achieved = byts / (top_ms * 1e-3) / 1e9
-        from bhgpu.fixed import tune_get
-        flux_k = "k_fx_flux_tile" if tune_get("mixed", "stage") else "k_fx_flux"
         kname = {"prims": "k_fx_c2p<float>", "ghosts": "k_fx_ghost<float>", "fluxes": f"{flux_k}<float,float,float>",
                  "update": "k_fx_update<float,float,float>"}[top]
         line = {
@@ -749,7 +759,7 @@ def run_ours(args):
                            "(interior cells' U and W rows 0-4, the blocks' own faces) from pinned host memory in and "
                            "out every step, unpacked and packed on the device",
                     "serial_value": world * zones / (ms_e2e_serial / 1e3), "serial_ms_per_step": ms_e2e_serial},
-            "gpu_launches": (LAUNCHES_PER_STEP + (2 if tune_get("mixed", "split") == 1 else 0)) * args.steps,
+            "gpu_launches": launches,
             "roofline": {"bound": "hbm", "kernel": f"{kname} ({top})", "achieved": achieved, "peak": peak,
                          "unit": "GB/s", "frac": achieved / peak,
                          "traffic": PROFILED_TRAFFIC.get(top) if args.grid == 128 else None,
