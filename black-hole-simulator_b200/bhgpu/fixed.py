@@ -127,8 +127,9 @@ class FxGrid:
                  persistent=False, nactive=None, maxlevel=None, tile_min=TILE_MIN):
         """emf_arrays: keep the edge EMFs in arrays (required, and the
         default, when blocks have different levels; otherwise they are
-        computed on the fly by the update).  persistent: launch the step
-        kernels as persistent CTAs fed by a device work queue.  nactive:
+        computed on the fly by the update).  persistent: launch
+        con2prim, fluxes, EMFs and update as persistent CTAs fed by a device
+        work queue.  nactive:
         the kernels work on blocks[:nactive] only (the rest are neighbours'
         copies, as in a sharded grid); maxlevel: the highest level of the
         whole domain (default: of these blocks); tile_min: the smallest

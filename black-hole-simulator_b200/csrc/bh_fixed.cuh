@@ -92,9 +92,9 @@ __device__ inline void atomic_max_pos(double* slot, double v) {
 // the item loop.  Without a queue, CTA t takes item t of the launch's work
 // list.  With one (the persistent form: a grid of resident CTAs), each CTA
 // starts with item blockIdx and takes further ones from a device counter until
-// none is left; the last CTA to
-// finish resets the counter for the next launch of the slot, so a step
-// needs no extra launch or memset and records into a CUDA graph as is.
+// none is left; the last CTA to finish resets the counter for the next launch
+// of the slot, so a step needs no extra launch or memset and records into a
+// CUDA graph as is.
 // ======================================================================
 struct Queue {
     int32_t* head;   // next item (NULL: one CTA per item)
@@ -855,7 +855,8 @@ __global__ void __launch_bounds__(FX_TPB, MINB) k_fx_update(FxPar P, Grid G, con
         // In FP64 everything read of the state goes out first: between the
         // stores a load waits for the store before it, which may alias, one
         // round trip to memory per variable (128^3, both halves, stages 0 and 1:
-        // 216 and 230 us at 4 CTAs per SM, before 266 and 272 at its best, 6).  The mixed variant keeps its order: the
+        // 197 and 212 us at 4 CTAs per SM, before 266 and 272 at its best, 6).  The
+        // mixed variant keeps its order: the
         // compiler contracts the FP32 source by it, and a step's roundings
         // are to stay (the fluxes' loads alone move without changing them).
         constexpr bool EARLY = sizeof(RT) == sizeof(double);
@@ -1279,7 +1280,7 @@ using FRT = BH_REAL;
 inline cudaStream_t fxs(void* s) { return (cudaStream_t)s; }
 inline int fx_launched() { return cudaGetLastError() == cudaSuccess ? BH_OK : BH_ECUDA; }
 // work-queue slots of the step kernels
-enum { QS_C2P = 0, QS_GHOST = 1, QS_FLUX = 2, QS_EMF = 3, QS_EMF_FIX = 4, QS_UPDATE = 5, QS_UPDATE_B = 6 };
+enum { QS_C2P = 0, QS_FLUX = 2, QS_EMF = 3, QS_UPDATE = 5, QS_UPDATE_B = 6 };   // (1 and 4: unused)
 static_assert(QS_UPDATE_B + 1 == BH_FX_QSLOTS, "queue slots");
 inline fx::Queue fx_q(const bh_fx_grid* g, int slot, int nitem) {
     if (!g->queue) return fx::Queue{nullptr, nullptr, nitem};

@@ -124,7 +124,7 @@ __global__ void k_ctop_pre(KP k, const double* U, const double* r, const double*
 // NaN where a feature is not finite.  The work per cell is nearly uniform,
 // so the CTA-wide steps of the network cost little; con2prim's own
 // iterations, whose count varies from cell to cell, run afterwards in
-// k_ctop_guess (one thread per cell, no barriers).
+// k_ctop (lanes refilled, no barriers).
 __global__ void __launch_bounds__(bh_tc::ROWS, 4)
     k_guess_tc(KP k, const __nv_bfloat16* wb, const float* norm, const double* U, const double* r,
                const double* th, int64_t n, double* xi0_out, int32_t* err) {

@@ -447,11 +447,13 @@ typedef struct bh_fx_grid {
     int32_t queue_ctas;          /* CTAs of a persistent launch (0: the SMs times the
                                     CTAs the kernel keeps resident per SM)          */
     int32_t *queue;              /* device [2 * BH_FX_QSLOTS], zeroed once before the
-                                    first launch, or NULL.  Set: every step kernel is
-                                    launched persistent, its CTAs taking work items
-                                    from a counter in this array (the counters reset
-                                    themselves at the end of each launch).  NULL: one
-                                    CTA per work item.  Both give the same results. */
+                                    first launch, or NULL.  Set: con2prim, fluxes, EMFs
+                                    and update are launched persistent, their CTAs
+                                    taking work items from a counter in this array
+                                    (the counters reset themselves at the end of each
+                                    launch); the ghost fill and the EMF correction
+                                    launch one CTA per work item all the same.  NULL:
+                                    so do all.  Both give the same results.         */
     const int32_t *items_flux;   /* device [nitem_flux][2] (block, e), or NULL/0: the work
                                     of the staged flux kernel.  e >= 0: tile e of the
                                     block's position box [-1, n]^3, tiles of 4 x 4 x 8
@@ -474,13 +476,14 @@ typedef struct bh_fx_grid {
                                     be there where they are more than items_pos, which
                                     tiles that fit their blocks exactly are not)    */
 } bh_fx_grid;
-#define BH_FX_QSLOTS 7
+#define BH_FX_QSLOTS 7          /* (two of them unused)                            */
 
 /* Launch bounds of the scheme's three heavy kernels (no counterpart in the
  * reference): each is compiled for 1 (no register cap) and 3 to 8
  * resident 128-thread CTAs per SM; the choice is per process and variant,
  * initially 0: by the library's rules, which follow the variant, the limiter
- * and the grid.  BH_FX_TUNE_STAGE (0, 1, or 2, initially 2: by rule) selects
+ * and the grid (bh_fx_tune_choice says what they give; bh_fx_tune_get returns
+ * the setting, so 0 or, for the next two, 2 where nothing else was set).  BH_FX_TUNE_STAGE (0, 1, or 2, initially 2: by rule) selects
  * the flux kernel: 1 = the stencil staged in shared memory per tile
  * (items_flux; grids without items_flux keep the unstaged kernel), with the
  * launch bounds of BH_FX_TUNE_FLUX.  BH_FX_TUNE_SPLIT (0, 1, or 2, initially
