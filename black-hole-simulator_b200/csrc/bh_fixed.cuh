@@ -1378,9 +1378,12 @@ namespace {
 //             1082 -> 801): more would spill.
 //   update    8 in FP32, 4 in FP64 (whose early loads fill the registers); as
 //             its two kernels with edge EMFs in arrays (lev 249 -> 210 / 249 ->
-//             248) and on grids of 8192 items, in FP64 2048, or more (128^3
-//             169 -> 166 a stage / 255 -> 223, 64^3 40 -> 38; below that the
-//             second launch costs more: 16^3 12 -> 17).
+//             248) and where one kernel takes more than one full wave in FP64
+//             (4 items per SM), two in FP32 (16 per SM): below that the second
+//             launch costs more than it saves.  Step split / whole, FP64 (FMA
+//             alike): 32^3 (256 items) 1.03, 36^3 (365) 1.01, 40^3 (500) 1.01,
+//             44^3 (666) .97, 48^3 .97, 64^3 .93, 128^3 .92; mixed: 48^3 (864)
+//             1.02, 64^3 (2048) 1.00, 68^3 (2457) .97, 80^3 .97, 128^3 .98.
 // A grid whose items are all resident at once without a cap takes none: nothing
 // waits for a slot, and a capped kernel's spills only lengthen it.  In FP64 the
 // uncapped kernels (172 to 246 registers) keep 2 CTAs per SM: step uncapped /
@@ -1412,7 +1415,7 @@ int fx_choose(int kernel, const bh_fx_params* P, const bh_fx_grid* g) {
     switch (kernel) {
     case BH_FX_TUNE_STAGE: return staged && g->nitem_flux && P->limiter != fx::FX_PPM;
     case BH_FX_TUNE_SPLIT:
-        return set != FX_AUTO_FORM ? set : (g->E || cell >= (F32 ? 8192 : 2048));
+        return set != FX_AUTO_FORM ? set : (g->E || cell > (F32 ? 16 : 4) * fx_sms());
     case BH_FX_TUNE_C2P: return set != FX_AUTO ? set : (cell <= few ? 1 : (F32 ? 7 : 6));
     case BH_FX_TUNE_FLUX:
         if (set != FX_AUTO) return set;

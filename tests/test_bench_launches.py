@@ -17,7 +17,7 @@ def bench():
     return m
 
 
-@pytest.mark.parametrize("n,launches,kernel", [(128, 11, "k_fx_flux_tile"), (64, 9, "k_fx_flux")])
+@pytest.mark.parametrize("n,launches,kernel", [(128, 11, "k_fx_flux_tile"), (8, 9, "k_fx_flux")])
 def test_by_rule_and_by_knob(n, launches, kernel):
     from bhgpu import fixed as fx
 

@@ -74,6 +74,14 @@ def test_caps_where_the_uncapped_kernels_would_queue():
             assert (choice("c2p", prec, c), choice("flux", prec, c)) == (1, want[1])
 
 
+def test_two_update_kernels_where_one_takes_more_waves():
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count if torch.cuda.is_available() else 1
+    for prec, per_sm in (("mixed", 16), ("fp64", 4), ("fp64-fma", 4)):
+        for items, want in ((per_sm * sms, 0), (per_sm * sms + 1, 1)):
+            assert choice("split", prec, dict(cell=items, pos=items, flux=items, tile=0)) == want
+
+
 @pytest.mark.gpu
 def test_exact_tiles_take_the_staged_fluxes_with_the_same_bits():
     import torch
