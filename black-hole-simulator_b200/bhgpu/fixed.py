@@ -147,7 +147,8 @@ class FxGrid:
         act = blocks[:self.nactive]
         self.items = {k: torch.from_numpy(work_items(act, k, self.ghost_depth)).to(dev)
                       for k in ("cell", "pos", "ghost")}
-        self.items["flux"] = torch.from_numpy(flux_items(act, tile_min)).to(dev)
+        flux = flux_items(act, tile_min)
+        self.items["flux"] = torch.from_numpy(flux).to(dev)
         wdt = torch.float32 if params.precision == "mixed" else torch.float64
         N = self.ncell
         self.U = torch.zeros((8, N), dtype=torch.float64, device=dev)
@@ -165,7 +166,7 @@ class FxGrid:
             emf_arrays = self.maxlevel > 0
         self.E = torch.zeros((3, N), dtype=torch.float64, device=dev) if emf_arrays else None
         self.queue = torch.zeros(2 * QSLOTS, dtype=torch.int32, device=dev) if persistent else None
-        self._rule = (0, 0, 0, item_counts(act, tile_min)["tile"])
+        self._rule = (0, 0, 0, int(np.count_nonzero(flux[:, 1] >= 0)))
         self._tile_min = tile_min
         self._refresh()
 
