@@ -308,7 +308,8 @@ class FxGrid:
 
     # ---- the step as one CUDA graph -----------------------------------------
     def capture(self):
-        """Record one step (9 launches) as a CUDA graph on a side stream
+        """Record one step (9 launches, 11 with the update as two
+        kernels, and those of levels) as a CUDA graph on a side stream
         (bh_fx_graph_create); ``replay()`` then runs a step with one launch
         of the graph.  The grid's buffers must not be reallocated while the
         graph lives."""

@@ -502,7 +502,8 @@ int bh_fx_tune_choice(const bh_fx_params *P, const bh_fx_grid *g, int32_t kernel
 
 /* one RK2 step: con2prim (+ CFL reduction), ghost fill, fluxes, update, twice */
 int bh_fx_step(const bh_fx_params *P, const bh_fx_grid *g, void *stream);
-/* bh_fx_step recorded once as a CUDA graph (9 launches; dt stays on the
+/* bh_fx_step recorded once as a CUDA graph (9 launches, 11 with the
+ * update as two kernels, and the passes and EMF kernels of levels; dt stays on the
  * device): replay and release it with bh_step_graph_replay / _destroy.
  * stream is required (not the legacy default stream); the grid's arrays
  * must stay valid at the same addresses while the graph lives. */
