@@ -855,10 +855,10 @@ __global__ void __launch_bounds__(FX_TPB, MINB) k_fx_update(FxPar P, Grid G, con
         // In FP64 everything read of the state goes out first: between the
         // stores a load waits for the store before it, which may alias, one
         // round trip to memory per variable (128^3, both halves, stages 0 and 1:
-        // 197 and 212 us at 4 CTAs per SM, before 266 and 272 at its best, 6).  The
-        // mixed variant keeps its order: the
-        // compiler contracts the FP32 source by it, and a step's roundings
-        // are to stay (the fluxes' loads alone move without changing them).
+        // 197 and 212 us at 4 CTAs per SM, before 266 and 272 at its best, 6).
+        // The mixed variant keeps its order: the compiler contracts the FP32
+        // source by it, and a step's roundings are to stay (the fluxes' loads
+        // alone move without changing them).
         constexpr bool EARLY = sizeof(RT) == sizeof(double);
         double u0[5], u1[5], b0[3], b1[3];
         FT div[5];
